@@ -128,8 +128,9 @@ constexpr int OZ_TX = 32, OZ_RJ = 8, OZ_KCH = 16;   // outer calvel/calmas z-mar
 // ---------------------------------------------------------------------------
 constexpr unsigned long long kMaxWaitNs = 2000000000ull;  // 2 s
 // ERR_WALL_LAW: a smooth-wall law did not converge; ERR_MID_BARRIER: a grid
-// barrier of the middle-level launch gave up waiting
-enum : int { ERR_TMA_WAIT = 1, ERR_WALL_LAW = 2, ERR_MID_BARRIER = 3 };
+// barrier of the middle-level launch gave up waiting; ERR_SIP_WAIT: a warp of
+// the SIP substitutions did for a neighbour's value
+enum : int { ERR_TMA_WAIT = 1, ERR_WALL_LAW = 2, ERR_MID_BARRIER = 3, ERR_SIP_WAIT = 4 };
 
 // Testing aid (mf3d_test_stall_copy): when nonzero, the first red-black
 // half-sweep CTA that sees it takes it (atomically, so exactly one CTA) and

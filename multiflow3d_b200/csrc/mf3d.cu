@@ -1856,8 +1856,9 @@ static int build_view(mf3d_ctx *C, View &V, const std::vector<DomainStore *> &do
 // V-cycle over a view.
 // ---------------------------------------------------------------------------
 template <typename T>
-static void halo(mf3d_ctx *C, View &V, int g, int q) {
+static void halo(mf3d_ctx *C, View &V, int g, int q, const int *act = nullptr) {
   ViewLevel &L = V.lv[g];
+  if (!act) act = V.act.p;
   if (!L.lmr_depth.empty()) {
     // LMR: the nodes depth by depth from the pre-exchange state, then the writes
     for (size_t d = 1; d < L.lmr_depth.size(); ++d) {
@@ -1878,11 +1879,11 @@ static void halo(mf3d_ctx *C, View &V, int g, int q) {
   T *buf = (T *)L.stage[q].p;
   if (L.n_staged[q]) {
     launch(k_halo_stage<T>, grid_of(L.n_staged[q], 256), 256, 0, C->stream, L.tab.p, L.hseg[q].p, L.n_hseg[q],
-                                                                       L.n_staged[q], V.act.p, buf);
+                                                                       L.n_staged[q], act, buf);
     ++C->launches;
   }
   launch(k_halo_apply<T>, grid_of(L.n_halo[q], 256), 256, 0, C->stream, L.tab.p, L.hseg[q].p, L.n_hseg[q],
-                                                                   L.n_halo[q], V.act.p, buf);
+                                                                   L.n_halo[q], act, buf);
   ++C->launches;
 }
 
