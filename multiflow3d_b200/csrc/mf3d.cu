@@ -934,9 +934,11 @@ struct View {
   std::vector<BlkFld> hf;
   DevBuf<BlkFld> df;
   DevBuf<Tile> t_int, t_zint, t_l1cells, t_faces, t_planes, t_pairs, t_vfaces;
-  DevBuf<Tile> t_bcax[3];             // bounds mode: 3 components x 2 faces x ttc plane per block, per axis
-  int n_bcax[3] = {0, 0, 0};
-  bool bc_periodic[3] = {false, false, false};  // some block has a periodic face along the axis
+  DevBuf<Tile> t_bcax[3], t_bcall;    // bounds mode: 2 faces x ttc plane per block, per axis; of all axes
+  int n_bcax[3] = {0, 0, 0}, n_bcall = 0;
+  // some block has along the axis: a periodic face alone, with a partner
+  // (BlkFld::pface 1, 2); a face without a neighbour
+  bool bc_alone[3] = {false, false, false}, bc_partner[3] = {false, false, false}, bc_wall[3] = {false, false, false};
   int n_pairs = 0, pairs_kch = 1;
   int n_int = 0, n_zint = 0, n_l1cells = 0, n_faces = 0, n_planes = 0, n_vfaces = 0;
   // field exchanges as copy maps (a view over one domain that has them):
@@ -1755,7 +1757,7 @@ static int build_view(mf3d_ctx *C, View &V, const std::vector<DomainStore *> &do
   // level-1 field tables
   V.hf.resize(nb);
   std::vector<Tile> t1, t2, t5;
-  std::vector<long long> it_faces, it_planes, it_vfaces, it_bcax[3];
+  std::vector<long long> it_faces, it_planes, it_vfaces, it_bcax[3], it_bcall;
   for (int b = 0; b < nb; ++b) {
     const BlockStore &S = *V.blk[b];
     BlkFld F = S.fld;
@@ -1779,10 +1781,15 @@ static int build_view(mf3d_ctx *C, View &V, const std::vector<DomainStore *> &do
     it_vfaces.push_back((long long)(C->prm.pl_ex + 1) * it_faces.back());
     {
       const long long ti = x.nx + 2 * (long long)F.pl, tj = x.ny + 2 * (long long)F.pl, tk = x.nz + 2 * (long long)F.pl;
-      it_bcax[0].push_back(6 * tj * tk);
-      it_bcax[1].push_back(6 * ti * tk);
-      it_bcax[2].push_back(6 * ti * tj);
-      for (int f = 0; f < 6; ++f) V.bc_periodic[f / 2] |= F.pface[f] != 0;
+      it_bcax[0].push_back(2 * tj * tk);
+      it_bcax[1].push_back(2 * ti * tk);
+      it_bcax[2].push_back(2 * ti * tj);
+      it_bcall.push_back(2 * (tj * tk + ti * tk + ti * tj));
+      for (int f = 0; f < 6; ++f) {
+        V.bc_alone[f / 2] |= F.pface[f] == 1;
+        V.bc_partner[f / 2] |= F.pface[f] == 2;
+        V.bc_wall[f / 2] |= F.wall[f] != 0;
+      }
     }
     V.n_l1 += (long long)x.nx * x.ny * x.nz;
   }
@@ -1813,6 +1820,11 @@ static int build_view(mf3d_ctx *C, View &V, const std::vector<DomainStore *> &do
       V.n_bcax[a] = (int)tb.size();
       if ((st = V.t_bcax[a].upload(tb, s))) return st;
     }
+  if (C->prm.bounds) {
+    auto tb = make_tiles(it_bcall);
+    V.n_bcall = (int)tb.size();
+    if ((st = V.t_bcall.upload(tb, s))) return st;
+  }
   if ((st = coarse_cycle_plan(C, V))) return st;
   if ((st = mid_cycle_plan(C, V))) return st;
   V.fx_uvw = V.fx_p = V.fxe_sub = V.fxe_chain = nullptr;
@@ -2631,15 +2643,28 @@ static bool bounds_code_unsupported(int f, int code, bool lsm, int alfabc, bool 
   return false;
 }
 
-// exchange_bc of u, v, w (only >= 0: of that component alone)
+// exchange_bc of u, v, w (only >= 0: of that component alone).  With a
+// partner behind every periodic face a layer is two launches, packs and
+// unpacks of all axes; else a launch per walk and axis that has work in it.
 static void bc_walks(mf3d_ctx *C, View &V, int only = -1) {
-  for (int ly = 0; ly <= C->prm.pl_ex; ++ly)
+  const unsigned comps = only >= 0 ? 1 : 3;
+  auto walk = [&](int a, int ly, int mode) {
+    launch(k_bc_walk, dim3(a < 0 ? V.n_bcall : V.n_bcax[a], comps), kTile, 0, C->stream, V.df.p,
+           a < 0 ? V.t_bcall.p : V.t_bcax[a].p, V.ds.p, a, ly, mode, only);
+    ++C->launches;
+  };
+  const bool alone = V.bc_alone[0] || V.bc_alone[1] || V.bc_alone[2];
+  const bool partner = V.bc_partner[0] || V.bc_partner[1] || V.bc_partner[2];
+  for (int ly = 0; ly <= C->prm.pl_ex; ++ly) {
+    if (!alone && partner) {
+      walk(-1, ly, 1);
+      walk(-1, ly, 2);
+      continue;
+    }
     for (int mode = 0; mode < 3; ++mode)
-      for (int a = 0; a < 3; ++a) {
-        if (!V.bc_periodic[a]) continue;
-        launch(k_bc_walk, V.n_bcax[a], kTile, 0, C->stream, V.df.p, V.t_bcax[a].p, V.ds.p, a, ly, mode, only);
-        ++C->launches;
-      }
+      for (int a = 0; a < 3; ++a)
+        if ((mode < 2 && V.bc_alone[a]) || (mode > 0 && V.bc_partner[a])) walk(a, ly, mode);
+  }
 }
 // the faces without a neighbour by their code, layers 0..pl_ex (only as above);
 // dt < 0: the solve's dt and alfapr.  The wall functions of a tangential
@@ -2647,13 +2672,14 @@ static void bc_walks(mf3d_ctx *C, View &V, int only = -1) {
 static void bound_faces(mf3d_ctx *C, View &V, int alfabc, int only = -1, double dt = 0.0, double alfapr = 0.0) {
   for (int ly = 0; ly <= C->prm.pl_ex; ++ly)
     for (int a = 0; a < 3; ++a) {
+      if (!V.bc_wall[a]) continue;
       if (V.wall_law && ly == 0 && only >= 0 && only != a) {
         launch(k_wall_law, V.n_bcax[a], kTile, 0, C->stream, V.df.p, V.t_bcax[a].p, V.ds.p, a, C->wall_re,
                C->wall_fric, V.err.p);
         ++C->launches;
       }
-      launch(k_bound_faces, V.n_bcax[a], kTile, 0, C->stream, V.df.p, V.t_bcax[a].p, V.ds.p, a, ly, C->prm.ubulk,
-             alfabc, only, dt, alfapr);
+      launch(k_bound_faces, dim3(V.n_bcax[a], only >= 0 ? 1 : 3), kTile, 0, C->stream, V.df.p, V.t_bcax[a].p, V.ds.p, a,
+             ly, C->prm.ubulk, alfabc, only, dt, alfapr);
       ++C->launches;
     }
 }
@@ -2700,6 +2726,21 @@ static int solve_end(mf3d_ctx *C, View &V) {
     }
   }
   return MF3D_OK;
+}
+
+// The predictor of component COMP by the context's differencing; mode: quo's.
+template <int COMP>
+static void predict(mf3d_ctx *C, View &V, int mode, double dt, double alfapr, int pforce, double forcn) {
+  const dim3 cta(RW_TX, RW_RJ);
+  if (C->prm.differencing == 2)  // 24*h and 12*h*h are never powers of two
+    launch(mode ? k_rk4th<COMP, 1> : k_rk4th<COMP, 0>, V.n_int, cta, 0, C->stream, V.df.p, V.t_int.p, dt, alfapr, pforce,
+           forcn);
+  else if (C->prm.differencing == 3)
+    launch(mode == 2 ? k_rkweno<COMP, 2> : mode ? k_rkweno<COMP, 1> : k_rkweno<COMP, 0>, V.n_int, cta, 0, C->stream,
+           V.df.p, V.t_int.p, C->prm.pl_ex, dt, alfapr, pforce, forcn);
+  else
+    launch(mode == 2 ? k_rk2nd<COMP, 2> : mode ? k_rk2nd<COMP, 1> : k_rk2nd<COMP, 0>, V.n_int, cta, 0, C->stream, V.df.p,
+           V.t_int.p, dt, alfapr, pforce, forcn);
 }
 
 // A kernel that gave up waiting (a TMA copy that never landed) leaves its
@@ -3663,19 +3704,26 @@ int mf3d_rungek_2nd_device(mf3d_ctx *C, const mf3d_fields *fields, const mf3d_rk
   cudaStream_t s = C->stream;
   C->launches = 0;
   CK(cudaMemsetAsync(V.ds.p, 0, V.ds.n * sizeof(DomState), s));  // no domain marked diverged
+  // how the stage's kernels divide by the spacings (quo): 2 every spacing a
+  // power of two, 1 by Markstein's correction (within 2^-40 .. 2^40, so that
+  // h*h, 12*h*h and 24*h are far inside its range), 0 otherwise
+  int mode = 2;
+  for (const auto &F : V.hf)
+    for (int a = 0; a < 3; ++a) {
+      const double h = a == 0 ? V.blk[&F - V.hf.data()]->d.dx : a == 1 ? V.blk[&F - V.hf.data()]->d.dy
+                                                                       : V.blk[&F - V.hf.data()]->d.dz;
+      if (!(h >= 0x1p-40 && h <= 0x1p+40)) mode = 0;
+      else if (F.pinv[a] == 0.0) mode = std::min(mode, 1);
+    }
   // rungek_conv2nd: boundu, the u loop, boundv, the v loop, boundw, the w
   // loop - each component's predictor sees the other components' ghosts as
   // they were before their own bound; rungek_diff2nd fused per component
   for (int comp = 0; comp < 3; ++comp) {
     bc_walks(C, V, comp);
     bound_faces(C, V, alfabc, comp, dt, alfapr);
-    if (C->prm.differencing == 2)
-      launch(k_rk4th, V.n_int, dim3(RW_TX, RW_RJ), 0, s, V.df.p, V.t_int.p, comp, dt, alfapr, pressureforce, forcn);
-    else if (C->prm.differencing == 3)
-      launch(k_rkweno, V.n_int, dim3(RW_TX, RW_RJ), 0, s, V.df.p, V.t_int.p, comp, C->prm.pl_ex, dt, alfapr,
-             pressureforce, forcn);
-    else
-      launch(k_rk2nd, V.n_int, dim3(RW_TX, RW_RJ), 0, s, V.df.p, V.t_int.p, comp, dt, alfapr, pressureforce, forcn);
+    if (comp == 0) predict<0>(C, V, mode, dt, alfapr, pressureforce, forcn);
+    else if (comp == 1) predict<1>(C, V, mode, dt, alfapr, pressureforce, forcn);
+    else predict<2>(C, V, mode, dt, alfapr, pressureforce, forcn);
     ++C->launches;
   }
   const cudaError_t e = cudaStreamSynchronize(s);

@@ -93,6 +93,25 @@ __global__ void k_selftest_divide(const double *x, const double *b, const double
   qref[t] = x[t] / b[t];
 }
 
+// x / b of a kernel that forms many quotients by the same b without a branch
+// each.  MODE 0 divides; 2: b is a power of two and rb its inverse (the
+// product rounds the exact quotient once); 1: Markstein's correction from
+// rb = RN(1/b), 2^-300 <= b <= 2^300.  It is the IEEE quotient for a normal x
+// of 2^-600 .. 2^600 (no step over- or underflows), the product x*rb is for
+// x = 0 (the signed zero); any other x sets `bad` and the caller divides its
+// cell again with MODE 0.
+template <int MODE>
+__device__ __forceinline__ double quo(double x, double b, double rb, bool &bad) {
+  if (MODE == 0) return x / b;
+  const double q0 = x * rb;
+  if (MODE == 2) return q0;
+  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+  const bool in = e - (1023u - 600u) <= 1200u;
+  bad |= !in && x != 0.0;
+  const double q1 = fma(fma(-b, q0, x), rb, q0);
+  return in ? fma(fma(-b, q1, x), rb, q1) : q0;
+}
+
 // x / b on an axis: EXACT when b is a power of two and rb its exact inverse.
 template <bool EXACT>
 __device__ __forceinline__ double qdiv(double x, double b, double rb) {
@@ -351,6 +370,27 @@ __device__ inline long long fidx_ax(const BlkFld &F, int ax, int a, int s, int t
   return ax == 0 ? fidx(F, a, s, t) : ax == 1 ? fidx(F, s, a, t) : fidx(F, s, t, a);
 }
 
+// Item q of the bounds tiles (two ttc face planes per axis): its side,
+// in-plane index q and local coordinates in the plane.  ax < 0: the tiles of
+// all three axes, x first, and ax is found; false past the last item.
+__device__ __forceinline__ bool bc_item(const BlkFld &F, int &ax, int &q, int &side, int &sl, int &tl) {
+  const int pl = F.pl;
+  for (int a = ax < 0 ? 0 : ax;; ++a) {
+    if (a > 2) return false;
+    const int m1 = (a == 0 ? F.ny : F.nx) + 2 * pl, m2 = (a == 2 ? F.ny : F.nz) + 2 * pl, plane = m1 * m2;
+    if (q < 2 * plane) {
+      ax = a;
+      side = q / plane;
+      q -= side * plane;
+      sl = q % m1 + 1 - pl;
+      tl = q / m1 + 1 - pl;
+      return true;
+    }
+    if (ax >= 0) return false;
+    q -= 2 * plane;
+  }
+}
+
 // One walk of exchange_bc (exchange_bc.for:16-838, every block on one
 // rank) over the two faces of axis `ax`, layer ly, full ghost-inclusive
 // planes.  mode 0: the first walk's self-copies of a block alone along the
@@ -361,25 +401,21 @@ __device__ inline long long fidx_ax(const BlkFld &F, int ax, int a, int s, int t
 // per layer as walk 1 for x, y, z, walk 2 for x, y, z, walk 3 for x, y, z:
 // a block's faces in the reference's W, E, S, N, B, T order.  Reads and
 // writes of one launch never meet (interior planes or receive planes
-// against ghost planes).  Items per block: 3 * 2 * n1 * n2 (ttc extents of
-// the other two axes).  Skipped after a diverged solve.
+// against ghost planes).  Where no block is alone along a periodic axis the
+// packs of all axes touch no ghost and run as one launch (ax = -1, mode 1),
+// and so do the unpacks (ax = -1, mode 2): a ghost that a later axis' unpack
+// writes too is left to it.  blockIdx.y: the component, or `only`.  Skipped
+// after a diverged solve.
 __global__ void k_bc_walk(const BlkFld *__restrict__ fl, const Tile *__restrict__ tiles,
                           const DomState *__restrict__ ds, int ax, int ly, int mode, int only) {
   pdl_wait();
   const Tile t = tiles[blockIdx.x];
   const BlkFld &F = fl[t.blk];
   if (ds[F.dom].rmax > 100.0) return;
-  const int pl = F.pl;
-  const int m1 = (ax == 0 ? F.ny : F.nx) + 2 * pl, m2 = (ax == 2 ? F.ny : F.nz) + 2 * pl;
-  int q = t.i0 + threadIdx.x;
-  const int plane = m1 * m2;
-  if (q >= 6 * plane) return;
-  const int comp = q / (2 * plane);
-  if (only >= 0 && comp != only) return;  // one component (boundu, boundv or boundw alone)
-  q -= comp * 2 * plane;
-  const int side = q / plane;
-  q -= side * plane;
-  const int sl = q % m1 + 1 - pl, tl = q / m1 + 1 - pl;  // local coordinates of the plane cell
+  const int comp = only >= 0 ? only : blockIdx.y;
+  const bool all = ax < 0;
+  int q = t.i0 + threadIdx.x, side, sl, tl;
+  if (!bc_item(F, ax, q, side, sl, tl)) return;
   const int f = 2 * ax + side;
   const int pf = F.pface[f];
   if (!pf) return;
@@ -387,6 +423,12 @@ __global__ void k_bc_walk(const BlkFld *__restrict__ fl, const Tile *__restrict_
   const int s0 = 1, e0 = comp_end(F, comp, ax);
   const long long g = fidx_ax(F, ax, side ? e0 + 1 + ly : s0 - 1 - ly, sl, tl);
   if (mode == 2) {
+    if (all) {
+      auto later = [&](int a, int x) {
+        return (F.pface[2 * a] == 2 && x == -ly) || (F.pface[2 * a + 1] == 2 && x == comp_end(F, comp, a) + 1 + ly);
+      };
+      if ((ax == 0 && later(1, sl)) || (ax < 2 && later(2, tl))) return;
+    }
     if (pf == 2) fi[g] = F.bcst[((long long)comp * 6 + f) * F.bcplane + q];
     return;
   }
@@ -510,16 +552,10 @@ __global__ void k_bound_faces(const BlkFld *__restrict__ fl, const Tile *__restr
   const BlkFld &F = fl[t.blk];
   if (ds[F.dom].rmax > 100.0) return;
   const int pl = F.pl;
-  const int m1 = (ax == 0 ? F.ny : F.nx) + 2 * pl, m2 = (ax == 2 ? F.ny : F.nz) + 2 * pl;
-  int q = t.i0 + threadIdx.x;
-  const int plane = m1 * m2;
-  if (q >= 6 * plane) return;
-  const int comp = q / (2 * plane);
-  if (only >= 0 && comp != only) return;  // one component (boundu, boundv or boundw alone)
-  q -= comp * 2 * plane;
-  const int side = q / plane;
-  q -= side * plane;
-  const int sl = q % m1 + 1 - pl, tl = q / m1 + 1 - pl;
+  const int m1 = (ax == 0 ? F.ny : F.nx) + 2 * pl;
+  const int comp = only >= 0 ? only : blockIdx.y;  // boundu, boundv or boundw alone, or all three
+  int q = t.i0 + threadIdx.x, side, sl, tl;
+  if (!bc_item(F, ax, q, side, sl, tl)) return;
   const int f = 2 * ax + side;
   if (!F.wall[f]) return;
   const int code = F.bcode[f];
@@ -1225,53 +1261,125 @@ __global__ void __launch_bounds__(RW_TX *RW_RJ) k_calmas4(const BlkFld *__restri
 //   u under pressureforce: star = star + dt*alfapr*forcn.
 // Fusing the two loops per cell keeps the reference's values: rungek_diff2nd
 // reads only the component itself, which boundv/boundw do not touch.
-__global__ void __launch_bounds__(RW_TX *RW_RJ) k_rk2nd(const BlkFld *__restrict__ fl, const Tile *__restrict__ tiles,
-                                                        int comp, double dt, double alfapr, int pforce, double forcn) {
+// Written in fluxes: with F_b(c) = (Vb(c) + Vb(past the face))*(C(c) +
+// C(c + e_b)) the reference's second product of axis b is F_b(c - e_b), and
+// um12 is up12 at c - e_a (the sums commute), so the z fluxes are carried up
+// the march, like the component itself.  The next plane's operands load
+// while a plane is computed.  What bounds it: DRAM, 48 B a cell (the three
+// velocities, the start-of-step value, the viscosity, the predicted value).
+// 256^3 in 8 blocks: 193 us a component (4.2 TB/s), against 267 us with six
+// IEEE divisions a cell, every operand loaded anew and none ahead.
+template <int COMP>
+struct Rk2Plane {  // what a plane adds to the march at (i, j): C at the plane above, this plane's neighbours
+  double ct, cw, ce, cs, cn;  // C(k+1), C(i-1), C(i+1), C(j-1), C(j+1)
+  double a0, a1, b0, b1;      // first transverse axis: Vb(c), Vb(c+so), Vb(c-sb), Vb(c-sb+so)
+  double d0, d1, e0, e1;      // second transverse axis; z: d only (the flux below is carried)
+  double oo, vis;
+};
+template <int COMP, int MODE>
+__device__ __forceinline__ double rk2_cell(const Rk2Plane<COMP> &v, double cc, double cb, double &fz,
+                                           const double *h, const double *r, const double *hh,
+                                           const double *rr, double dt, double alfapr, int pforce, double forcn,
+                                           bool &bad) {
+  // fluxes of the three axes at the high and low side of the face
+  double hi[3], lo[3];
+  auto sq = [](double a, double b) { const double m = 0.5 * (a + b); return m * m; };
+  if (COMP == 0) {
+    hi[0] = sq(cc, v.ce); lo[0] = sq(cc, v.cw);
+    hi[1] = (v.a0 + v.a1) * (cc + v.cn); lo[1] = (v.b0 + v.b1) * (cc + v.cs);
+    hi[2] = (v.d0 + v.d1) * (cc + v.ct);
+  } else if (COMP == 1) {
+    hi[0] = (v.a0 + v.a1) * (cc + v.ce); lo[0] = (v.b0 + v.b1) * (cc + v.cw);
+    hi[1] = sq(cc, v.cn); lo[1] = sq(cc, v.cs);
+    hi[2] = (v.d0 + v.d1) * (cc + v.ct);
+  } else {
+    hi[0] = (v.a0 + v.a1) * (cc + v.ce); lo[0] = (v.b0 + v.b1) * (cc + v.cw);
+    hi[1] = (v.d0 + v.d1) * (cc + v.cn); lo[1] = (v.e0 + v.e1) * (cc + v.cs);
+    hi[2] = sq(cc, v.ct);
+  }
+  lo[2] = fz;
+  fz = hi[2];
+  double c[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const double d = hi[a] - lo[a];
+    c[a] = quo<MODE>(a == COMP ? d : 0.25 * d, h[a], r[a], bad);
+  }
+  double st = (v.oo - dt * alfapr * (c[0] + c[1] + c[2]));
+  const double aw = quo<MODE>(-v.vis, hh[0], rr[0], bad), as = quo<MODE>(-v.vis, hh[1], rr[1], bad),
+               ab = quo<MODE>(-v.vis, hh[2], rr[2], bad);
+  const double ap = -1.0 * (aw + aw + as + as + ab + ab);
+  const double diff = -(ap * cc + as * v.cn + as * v.cs + aw * v.ce + aw * v.cw + ab * v.ct + ab * cb);
+  st = (st + dt * alfapr * diff);
+  if (COMP == 0 && pforce) st = st + dt * alfapr * forcn;
+  return st;
+}
+template <int COMP, int MODE>
+__global__ void __launch_bounds__(RW_TX *RW_RJ, 3) k_rk2nd(const BlkFld *__restrict__ fl,
+                                                           const Tile *__restrict__ tiles, double dt, double alfapr,
+                                                           int pforce, double forcn) {
   pdl_wait();
   const Tile t = tiles[blockIdx.x];
   const BlkFld &F = fl[t.blk];
   const int i = t.i0 + threadIdx.x, j = t.j0 + threadIdx.y;
-  if (i > comp_end(F, comp, 0) || j > comp_end(F, comp, 1)) return;
-  const int k1 = min(t.k0 + RW_KCH - 1, comp_end(F, comp, 2));
+  if (i > comp_end(F, COMP, 0) || j > comp_end(F, COMP, 1)) return;
+  const int k1 = min(t.k0 + RW_KCH - 1, comp_end(F, COMP, 2));
+  if (t.k0 > k1) return;
   const long long sy = F.ti, sz = (long long)F.ti * F.tj;
-  const double dx = F.h[0][1], dy = F.h[1][1], dz = F.h[2][1];
-  const double dxx = dx * dx, dyy = dy * dy, dzz = dz * dz;
+  const double h[3] = {F.h[0][1], F.h[1][1], F.h[2][1]};
+  const double hh[3] = {h[0] * h[0], h[1] * h[1], h[2] * h[2]};
+  double r[3], rr[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    r[a] = MODE ? 1.0 / h[a] : 0.0;
+    rr[a] = MODE ? 1.0 / hh[a] : 0.0;
+  }
   const double *__restrict__ U = F.u;
   const double *__restrict__ V = F.v;
   const double *__restrict__ W = F.w;
-  const double *__restrict__ C = comp_field(F, comp);
-  const double *__restrict__ OO = F.oo[comp];
-  double *__restrict__ ST = comp == 0 ? F.ustar : comp == 1 ? F.vstar : F.wstar;
-  const long long so = comp == 0 ? 1 : comp == 1 ? sy : sz;  // the cell past the face
-  for (int k = t.k0; k <= k1; ++k) {
-    const long long c = fidx(F, i, j, k);
-    double c1, c2, c3;
-    if (comp == 0) {
-      const double up12 = 0.5 * (U[c] + U[c + 1]), um12 = 0.5 * (U[c] + U[c - 1]);
-      c1 = (up12 * up12 - um12 * um12) / dx;
-      c2 = 0.25 * ((V[c] + V[c + 1]) * (U[c] + U[c + sy]) - (V[c - sy] + V[c + 1 - sy]) * (U[c] + U[c - sy])) / dy;
-      c3 = 0.25 * ((W[c] + W[c + 1]) * (U[c] + U[c + sz]) - (W[c - sz] + W[c + 1 - sz]) * (U[c] + U[c - sz])) / dz;
-    } else if (comp == 1) {
-      const double vp12 = 0.5 * (V[c] + V[c + sy]), vm12 = 0.5 * (V[c] + V[c - sy]);
-      c2 = (vp12 * vp12 - vm12 * vm12) / dy;
-      c1 = 0.25 * ((U[c] + U[c + sy]) * (V[c] + V[c + 1]) - (U[c - 1] + U[c - 1 + sy]) * (V[c] + V[c - 1])) / dx;
-      c3 = 0.25 * ((W[c] + W[c + sy]) * (V[c] + V[c + sz]) - (W[c - sz] + W[c + sy - sz]) * (V[c] + V[c - sz])) / dz;
+  const double *__restrict__ C = COMP == 0 ? F.u : COMP == 1 ? F.v : F.w;
+  const double *__restrict__ OO = F.oo[COMP];
+  const double *__restrict__ VIS = F.vis;
+  double *__restrict__ ST = COMP == 0 ? F.ustar : COMP == 1 ? F.vstar : F.wstar;
+  const long long so = COMP == 0 ? 1 : COMP == 1 ? sy : sz;  // the cell past the face
+  auto load = [&](long long c) {
+    Rk2Plane<COMP> v;
+    v.ct = C[c + sz]; v.cw = C[c - 1]; v.ce = C[c + 1]; v.cs = C[c - sy]; v.cn = C[c + sy];
+    if (COMP == 0) {
+      v.a0 = V[c]; v.a1 = V[c + 1]; v.b0 = V[c - sy]; v.b1 = V[c + 1 - sy];
+      v.d0 = W[c]; v.d1 = W[c + 1];
+    } else if (COMP == 1) {
+      v.a0 = U[c]; v.a1 = U[c + sy]; v.b0 = U[c - 1]; v.b1 = U[c - 1 + sy];
+      v.d0 = W[c]; v.d1 = W[c + sy];
     } else {
-      const double wp12 = 0.5 * (W[c] + W[c + sz]), wm12 = 0.5 * (W[c] + W[c - sz]);
-      c3 = (wp12 * wp12 - wm12 * wm12) / dz;
-      c1 = 0.25 * ((U[c] + U[c + sz]) * (W[c] + W[c + 1]) - (U[c - 1] + U[c - 1 + sz]) * (W[c] + W[c - 1])) / dx;
-      c2 = 0.25 * ((V[c] + V[c + sz]) * (W[c] + W[c + sy]) - (V[c - sy] + V[c - sy + sz]) * (W[c] + W[c - sy])) / dy;
+      v.a0 = U[c]; v.a1 = U[c + sz]; v.b0 = U[c - 1]; v.b1 = U[c - 1 + sz];
+      v.d0 = V[c]; v.d1 = V[c + sz]; v.e0 = V[c - sy]; v.e1 = V[c - sy + sz];
     }
-    double st = (OO[c] - dt * alfapr * (c1 + c2 + c3));
-    const double visc = F.vis[c + so];
-    const double aw = -visc / dxx, ae = -visc / dxx, an = -visc / dyy, as = -visc / dyy;
-    const double at = -visc / dzz, ab = -visc / dzz;
-    const double ap = -1.0 * (aw + ae + as + an + ab + at);
-    const double diff = -(ap * C[c] + an * C[c + sy] + as * C[c - sy] + ae * C[c + 1] + aw * C[c - 1] +
-                          at * C[c + sz] + ab * C[c - sz]);
-    st = (st + dt * alfapr * diff);
-    if (comp == 0 && pforce) st = st + dt * alfapr * forcn;
+    v.oo = OO[c]; v.vis = VIS[c + so];
+    return v;
+  };
+  const long long c0 = fidx(F, i, j, t.k0);
+  double cc = C[c0], cb = C[c0 - sz];
+  // the z flux below the first plane
+  const double m = 0.5 * (cc + cb);
+  double fz = COMP == 2 ? m * m
+                        : (COMP == 0 ? W[c0 - sz] + W[c0 + 1 - sz] : W[c0 - sz] + W[c0 + sy - sz]) * (cc + cb);
+  Rk2Plane<COMP> v = load(c0);
+  for (int k = t.k0; k <= k1; ++k) {
+    const long long c = c0 + (k - t.k0) * sz;
+    Rk2Plane<COMP> nx = v;
+    if (k < k1) nx = load(c + sz);
+    bool bad = false;
+    const double below = fz;
+    double st = rk2_cell<COMP, MODE>(v, cc, cb, fz, h, r, hh, rr, dt, alfapr, pforce, forcn, bad);
+    if (MODE == 1 && bad) {
+      double f = below;
+      st = rk2_cell<COMP, 0>(v, cc, cb, f, h, r, hh, rr, dt, alfapr, pforce, forcn, bad);
+    }
     ST[c] = st;
+    cb = cc;
+    cc = v.ct;
+    v = nx;
   }
 }
 
@@ -1290,71 +1398,86 @@ __global__ void __launch_bounds__(RW_TX *RW_RJ) k_rk2nd(const BlkFld *__restrict
 //     face for v and w (rungek.for:230, 262, 290);
 //   u under pressureforce: star = star + dt*alfapr*forcn.
 // The stencils reach three cells each way (pl >= 3).
-__global__ void __launch_bounds__(RW_TX *RW_RJ) k_rk4th(const BlkFld *__restrict__ fl, const Tile *__restrict__ tiles,
-                                                        int comp, double dt, double alfapr, int pforce, double forcn) {
-  pdl_wait();
-  const Tile t = tiles[blockIdx.x];
-  const BlkFld &F = fl[t.blk];
-  const int i = t.i0 + threadIdx.x, j = t.j0 + threadIdx.y;
-  if (i > comp_end(F, comp, 0) || j > comp_end(F, comp, 1)) return;
-  const int k1 = min(t.k0 + RW_KCH - 1, comp_end(F, comp, 2));
-  const long long st3[3] = {1, (long long)F.ti, (long long)F.ti * F.tj};
-  const double h[3] = {F.h[0][1], F.h[1][1], F.h[2][1]};
-  const double *vel[3] = {F.u, F.v, F.w};
-  const double *__restrict__ Cf = vel[comp];
-  const double *__restrict__ OO = F.oo[comp];
-  double *__restrict__ ST = comp == 0 ? F.ustar : comp == 1 ? F.vstar : F.wstar;
-  const long long sa = st3[comp];
+// What bounds it: loads through L1 (54 operands a cell) and issue.  COMP
+// fixes the strides' roles at compile time (no indexing of local arrays) and
+// the six quotients take quo: 4 blocks of 90x117x75, 97-113 us a component
+// against 132 us.
+template <int COMP, int MODE>
+__device__ __forceinline__ double rk4_cell(const double *const *vel, const double *OO, const double *VIS,
+                                           const long long *st3, const double *h24, const double *r24,
+                                           const double *h12, const double *r12, long long c, double dt,
+                                           double alfapr, int pforce, double forcn, bool &bad) {
+  const double *Cf = vel[COMP];
+  const long long sa = st3[COMP];
   // (-f(+1) + 9 f(0) + 9 f(-1) - f(-2)) / 16 along stride s, around element e
   auto q4 = [](const double *f, long long e, long long s) {
     return (-f[e + s] + 9.0 * f[e] + 9.0 * f[e - s] - f[e - 2 * s]) / 16.0;
   };
-  auto d4 = [](double p1, double p0, double m1, double m2, double hh) {
-    return (-p1 + 27.0 * p0 - 27.0 * m1 + m2) / (24.0 * hh);
-  };
-  for (int k = t.k0; k <= k1; ++k) {
-    const long long c = fidx(F, i, j, k);
-    double term[3];
+  double term[3], lap[3];
 #pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      if (b == comp) {
-        double s4[4];
+  for (int b = 0; b < 3; ++b) {
+    const long long sb = st3[b];
+    double p4[4];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const double q = q4(Cf, c + (2 - m) * sa, sa);
-          s4[m] = q * q;
-        }
-        term[b] = d4(s4[0], s4[1], s4[2], s4[3], h[b]);
+    for (int m = 0; m < 4; ++m) {
+      if (b == COMP) {
+        const double q = q4(Cf, c + (2 - m) * sa, sa);
+        p4[m] = q * q;
       } else {
-        const long long sb = st3[b];
-        double p4[4];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const long long e = c + (1 - m) * sb;  // b-offset 1, 0, -1, -2
-          p4[m] = q4(Cf, e + sb, sb) * q4(vel[b], e + sa, sa);
-        }
-        term[b] = d4(p4[0], p4[1], p4[2], p4[3], h[b]);
+        const long long e = c + (1 - m) * sb;  // b-offset 1, 0, -1, -2
+        p4[m] = q4(Cf, e + sb, sb) * q4(vel[b], e + sa, sa);
       }
     }
-    double st = (OO[c] - dt * alfapr * (term[0] + term[1] + term[2]));
-    const double visc = F.vis[comp == 0 ? c : c + sa];
-    double lap[3];
+    term[b] = quo<MODE>(-p4[0] + 27.0 * p4[1] - 27.0 * p4[2] + p4[3], h24[b], r24[b], bad);
+    lap[b] = quo<MODE>(-Cf[c + 2 * sb] + 16.0 * Cf[c + sb] - 30.0 * Cf[c] + 16.0 * Cf[c - sb] - Cf[c - 2 * sb], h12[b],
+                       r12[b], bad);
+  }
+  double st = (OO[c] - dt * alfapr * (term[0] + term[1] + term[2]));
+  const double visc = VIS[COMP == 0 ? c : c + sa];
+  const double diff = visc * (lap[0] + lap[1] + lap[2]);
+  st = (st + dt * alfapr * diff);
+  if (COMP == 0 && pforce) st = st + dt * alfapr * forcn;
+  return st;
+}
+template <int COMP, int MODE>
+__global__ void __launch_bounds__(RW_TX *RW_RJ, 2) k_rk4th(const BlkFld *__restrict__ fl,
+                                                           const Tile *__restrict__ tiles, double dt, double alfapr,
+                                                           int pforce, double forcn) {
+  pdl_wait();
+  const Tile t = tiles[blockIdx.x];
+  const BlkFld &F = fl[t.blk];
+  const int i = t.i0 + threadIdx.x, j = t.j0 + threadIdx.y;
+  if (i > comp_end(F, COMP, 0) || j > comp_end(F, COMP, 1)) return;
+  const int k1 = min(t.k0 + RW_KCH - 1, comp_end(F, COMP, 2));
+  const long long st3[3] = {1, (long long)F.ti, (long long)F.ti * F.tj};
+  const double *vel[3] = {F.u, F.v, F.w};
+  const double *__restrict__ OO = F.oo[COMP];
+  const double *__restrict__ VIS = F.vis;
+  double *__restrict__ ST = COMP == 0 ? F.ustar : COMP == 1 ? F.vstar : F.wstar;
+  double h24[3], r24[3], h12[3], r12[3];
 #pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      const long long sb = st3[b];
-      lap[b] = (-Cf[c + 2 * sb] + 16.0 * Cf[c + sb] - 30.0 * Cf[c] + 16.0 * Cf[c - sb] - Cf[c - 2 * sb]) /
-               (12.0 * (h[b] * h[b]));
-    }
-    const double diff = visc * (lap[0] + lap[1] + lap[2]);
-    st = (st + dt * alfapr * diff);
-    if (comp == 0 && pforce) st = st + dt * alfapr * forcn;
+  for (int a = 0; a < 3; ++a) {
+    const double h = F.h[a][1];
+    h24[a] = 24.0 * h;
+    h12[a] = 12.0 * (h * h);
+    r24[a] = MODE ? 1.0 / h24[a] : 0.0;
+    r12[a] = MODE ? 1.0 / h12[a] : 0.0;
+  }
+  for (int k = t.k0; k <= k1; ++k) {
+    const long long c = fidx(F, i, j, k);
+    bool bad = false;
+    double st = rk4_cell<COMP, MODE>(vel, OO, VIS, st3, h24, r24, h12, r12, c, dt, alfapr, pforce, forcn, bad);
+    if (MODE == 1 && bad)
+      st = rk4_cell<COMP, 0>(vel, OO, VIS, st3, h24, r24, h12, r12, c, dt, alfapr, pforce, forcn, bad);
     ST[c] = st;
   }
 }
 
 // HJ_WENO's fifth-order one-sided derivative from five divided differences
 // (weno.for:56-78; REAL is double, x**2 is x*x, MAX of the five squares).
-__device__ __forceinline__ double weno5(double v1, double v2, double v3, double v4, double v5) {
+// MODE as in quo: the three weights share the reciprocal of their sum.
+template <int MODE>
+__device__ __forceinline__ double weno5(double v1, double v2, double v3, double v4, double v5, bool &bad) {
   const double v11 = v1 * v1, v22 = v2 * v2, v33 = v3 * v3, v44 = v4 * v4, v55 = v5 * v5;
   const double e = (1.0E-6) * fmax(fmax(fmax(fmax(v11, v22), v33), v44), v55) + 1.0E-99;
   const double t11 = v1 - 2.0 * v2 + v3, t12 = v1 - 4.0 * v2 + 3.0 * v3;
@@ -1365,89 +1488,124 @@ __device__ __forceinline__ double weno5(double v1, double v2, double v3, double 
   const double S3 = (13.0 / 12.0) * (t31 * t31) + 0.25 * (t32 * t32);
   const double d1 = e + S1, d2 = e + S2, d3 = e + S3;
   const double a1 = 0.1 / (d1 * d1), a2 = 0.6 / (d2 * d2), a3 = 0.3 / (d3 * d3);
-  const double w1 = a1 / (a1 + a2 + a3), w2 = a2 / (a1 + a2 + a3), w3 = a3 / (a1 + a2 + a3);
+  const double sum = a1 + a2 + a3;
+  const double rs = MODE ? 1.0 / sum : 0.0;
+  if (MODE) bad |= !(sum >= 0x1p-300 && sum <= 0x1p+300);
+  constexpr int M = MODE ? 1 : 0;
+  const double w1 = quo<M>(a1, sum, rs, bad), w2 = quo<M>(a2, sum, rs, bad), w3 = quo<M>(a3, sum, rs, bad);
   return w1 * (v1 * (1.0 / 3.0) - v2 * (7.0 / 6.0) + v3 * (11.0 / 6.0)) +
          w2 * (-(v2 * (1.0 / 6.0)) + v3 * (5.0 / 6.0) + v4 * (1.0 / 3.0)) +
          w3 * (v3 * (1.0 / 3.0) + v4 * (5.0 / 6.0) - v5 * (1.0 / 6.0));
 }
 
 // The same stage with differencing = 3: rungek_convWENO (rungek.for:
-// 414-582) then rungek_diff2nd, for component `comp`.  Each derivative is
+// 414-582) then rungek_diff2nd, for component COMP.  Each derivative is
 // HJ_WENO's (weno.for:2-354) at this cell - the divided differences
 // D1(m) = (f(m+1) - f(m))/h formed on the fly - upwinded by the sign of the
 // advecting velocity (its own value along its axis, the 4-face average
 // 0.25*(...) along the others), 0 where that is 0; HJ_WENO leaves 0 outside
 // cells 4 .. end + pl_ex + 1 - 3 of each axis (1-based field indices; end
 // the component's range end), and so does this.  Then rungek_diff2nd's
-// terms as k_rk2nd forms them.
-__global__ void __launch_bounds__(RW_TX *RW_RJ) k_rkweno(const BlkFld *__restrict__ fl, const Tile *__restrict__ tiles,
-                                                         int comp, int pl_ex, double dt, double alfapr, int pforce,
-                                                         double forcn) {
+// terms as k_rk2nd forms them.  Issue bound: both upwind sides take one
+// evaluation on selected differences (a warp holds both signs), and the
+// quotients by h, h*h and the weights' sum need no division each (quo).
+// 128^3 in 8 blocks: 137 us a component against 268 us.
+template <int COMP, int MODE>
+__device__ __forceinline__ double rkw_cell(const double *U, const double *V, const double *W, const double *OO,
+                                           const double *VIS, const long long *st3, const int *fx, const int *lim,
+                                           const double *h, const double *r, const double *hh, const double *rr,
+                                           long long c, double dt, double alfapr, int pforce, double forcn,
+                                           bool &bad) {
+  const double *Cf = COMP == 0 ? U : COMP == 1 ? V : W;
+  const long long sy = st3[1], sz = st3[2];
+  // the advecting velocity of each axis at this face
+  double adv[3];
+  if (COMP == 0) {
+    adv[0] = U[c];
+    adv[1] = 0.25 * (V[c] + V[c + 1] + V[c - sy] + V[c + 1 - sy]);
+    adv[2] = 0.25 * (W[c] + W[c + 1] + W[c - sz] + W[c + 1 - sz]);
+  } else if (COMP == 1) {
+    adv[0] = 0.25 * (U[c] + U[c + sy] + U[c - 1] + U[c - 1 + sy]);
+    adv[1] = V[c];
+    adv[2] = 0.25 * (W[c] + W[c + sy] + W[c - sz] + W[c + sy - sz]);
+  } else {
+    adv[0] = 0.25 * (U[c] + U[c + sz] + U[c - 1] + U[c - 1 + sz]);
+    adv[1] = 0.25 * (V[c] + V[c + sz] + V[c - sy] + V[c - sy + sz]);
+    adv[2] = W[c];
+  }
+  double term[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const double sgn = adv[a];
+    double d = 0.0;
+    // HJ_WENO writes cells 4 .. lim-3 along a, 1 .. lim of the others
+    bool inside = fx[a] >= 4 && fx[a] <= lim[a] - 3;
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      if (b != a) inside = inside && fx[b] >= 1 && fx[b] <= lim[b];
+    if (inside && sgn != 0.0) {
+      const long long s = st3[a];
+      // plus (L = I = cell - 3): D1(+2) .. D1(-2); minus (L = I - 1): D1(-3) .. D1(+1)
+      const bool up = sgn > 0.0;
+      const double *f = Cf + c;
+      const long long o = up ? -3 * s : 3 * s, w = up ? s : -s;
+      double g[6];
+#pragma unroll
+      for (int m = 0; m < 6; ++m) g[m] = f[o + m * w];
+      // f(m+1) - f(m) in either direction
+      double dd[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m)
+        dd[m] = quo<MODE>(up ? g[m + 1] - g[m] : g[m] - g[m + 1], h[a], r[a], bad);
+      d = weno5<MODE>(dd[0], dd[1], dd[2], dd[3], dd[4], bad);
+    }
+    term[a] = sgn * d;
+  }
+  double st = (OO[c] - dt * alfapr * (term[0] + term[1] + term[2]));
+  const double visc = VIS[c + st3[COMP]];
+  const double aw = quo<MODE>(-visc, hh[0], rr[0], bad), as = quo<MODE>(-visc, hh[1], rr[1], bad),
+               ab = quo<MODE>(-visc, hh[2], rr[2], bad);
+  const double ap = -1.0 * (aw + aw + as + as + ab + ab);
+  const double diff = -(ap * Cf[c] + as * Cf[c + sy] + as * Cf[c - sy] + aw * Cf[c + 1] + aw * Cf[c - 1] +
+                        ab * Cf[c + sz] + ab * Cf[c - sz]);
+  st = (st + dt * alfapr * diff);
+  if (COMP == 0 && pforce) st = st + dt * alfapr * forcn;
+  return st;
+}
+template <int COMP, int MODE>
+__global__ void __launch_bounds__(RW_TX *RW_RJ, 2) k_rkweno(const BlkFld *__restrict__ fl,
+                                                            const Tile *__restrict__ tiles, int pl_ex, double dt,
+                                                            double alfapr, int pforce, double forcn) {
   pdl_wait();
   const Tile t = tiles[blockIdx.x];
   const BlkFld &F = fl[t.blk];
   const int i = t.i0 + threadIdx.x, j = t.j0 + threadIdx.y;
-  if (i > comp_end(F, comp, 0) || j > comp_end(F, comp, 1)) return;
-  const int k1 = min(t.k0 + RW_KCH - 1, comp_end(F, comp, 2));
+  if (i > comp_end(F, COMP, 0) || j > comp_end(F, COMP, 1)) return;
+  const int k1 = min(t.k0 + RW_KCH - 1, comp_end(F, COMP, 2));
   const long long st3[3] = {1, (long long)F.ti, (long long)F.ti * F.tj};
-  const double h[3] = {F.h[0][1], F.h[1][1], F.h[2][1]};
   const double *__restrict__ U = F.u;
   const double *__restrict__ V = F.v;
   const double *__restrict__ W = F.w;
-  const double *__restrict__ Cf = comp_field(F, comp);
-  const double *__restrict__ OO = F.oo[comp];
-  double *__restrict__ ST = comp == 0 ? F.ustar : comp == 1 ? F.vstar : F.wstar;
-  // HJ_WENO's range ends, 1-based field indices: the component's ends + pl_ex + 1
-  int lim[3];
+  const double *__restrict__ OO = F.oo[COMP];
+  const double *__restrict__ VIS = F.vis;
+  double *__restrict__ ST = COMP == 0 ? F.ustar : COMP == 1 ? F.vstar : F.wstar;
+  double h[3], r[3], hh[3], rr[3];
+  int lim[3];  // HJ_WENO's range ends, 1-based field indices: the component's ends + pl_ex + 1
 #pragma unroll
-  for (int a = 0; a < 3; ++a) lim[a] = comp_end(F, comp, a) + F.pl + pl_ex + 1;
-  const long long sy = st3[1], sz = st3[2];
+  for (int a = 0; a < 3; ++a) {
+    h[a] = F.h[a][1];
+    hh[a] = h[a] * h[a];
+    r[a] = MODE ? 1.0 / h[a] : 0.0;
+    rr[a] = MODE ? 1.0 / hh[a] : 0.0;
+    lim[a] = comp_end(F, COMP, a) + F.pl + pl_ex + 1;
+  }
   for (int k = t.k0; k <= k1; ++k) {
     const long long c = fidx(F, i, j, k);
     const int fx[3] = {i + F.pl, j + F.pl, k + F.pl};  // 1-based field indices
-    // the advecting velocity of each axis at this face
-    double adv[3];
-    if (comp == 0) {
-      adv[0] = U[c];
-      adv[1] = 0.25 * (V[c] + V[c + 1] + V[c - sy] + V[c + 1 - sy]);
-      adv[2] = 0.25 * (W[c] + W[c + 1] + W[c - sz] + W[c + 1 - sz]);
-    } else if (comp == 1) {
-      adv[0] = 0.25 * (U[c] + U[c + sy] + U[c - 1] + U[c - 1 + sy]);
-      adv[1] = V[c];
-      adv[2] = 0.25 * (W[c] + W[c + sy] + W[c - sz] + W[c + sy - sz]);
-    } else {
-      adv[0] = 0.25 * (U[c] + U[c + sz] + U[c - 1] + U[c - 1 + sz]);
-      adv[1] = 0.25 * (V[c] + V[c + sz] + V[c - sy] + V[c - sy + sz]);
-      adv[2] = W[c];
-    }
-    double term[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double sgn = adv[a];
-      double d = 0.0;
-      // HJ_WENO writes cells 4 .. lim-3 along a, 1 .. lim of the others
-      bool inside = fx[a] >= 4 && fx[a] <= lim[a] - 3;
-#pragma unroll
-      for (int b = 0; b < 3; ++b)
-        if (b != a) inside = inside && fx[b] >= 1 && fx[b] <= lim[b];
-      if (inside && sgn != 0.0) {
-        const long long s = st3[a];
-        auto D1 = [&](int m) { return (Cf[c + (m + 1) * s] - Cf[c + m * s]) / h[a]; };
-        // plus (L = I = cell - 3): D1(+2) .. D1(-2); minus (L = I - 1): D1(-3) .. D1(+1)
-        d = sgn > 0.0 ? weno5(D1(-3), D1(-2), D1(-1), D1(0), D1(1)) : weno5(D1(2), D1(1), D1(0), D1(-1), D1(-2));
-      }
-      term[a] = sgn * d;
-    }
-    double st = (OO[c] - dt * alfapr * (term[0] + term[1] + term[2]));
-    const double dxx = h[0] * h[0], dyy = h[1] * h[1], dzz = h[2] * h[2];
-    const double visc = F.vis[c + st3[comp]];
-    const double aw = -visc / dxx, ae = -visc / dxx, an = -visc / dyy, as = -visc / dyy;
-    const double at = -visc / dzz, ab = -visc / dzz;
-    const double ap = -1.0 * (aw + ae + as + an + ab + at);
-    const double diff = -(ap * Cf[c] + an * Cf[c + sy] + as * Cf[c - sy] + ae * Cf[c + 1] + aw * Cf[c - 1] +
-                          at * Cf[c + sz] + ab * Cf[c - sz]);
-    st = (st + dt * alfapr * diff);
-    if (comp == 0 && pforce) st = st + dt * alfapr * forcn;
+    bool bad = false;
+    double st = rkw_cell<COMP, MODE>(U, V, W, OO, VIS, st3, fx, lim, h, r, hh, rr, c, dt, alfapr, pforce, forcn, bad);
+    if (MODE && bad)
+      st = rkw_cell<COMP, 0>(U, V, W, OO, VIS, st3, fx, lim, h, r, hh, rr, c, dt, alfapr, pforce, forcn, bad);
     ST[c] = st;
   }
 }
