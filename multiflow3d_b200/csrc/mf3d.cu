@@ -107,6 +107,10 @@ static bool injected_alloc_failure() {
   return c == 0;
 }
 
+// Testing aid (mf3d_test_stall_copy): set while a stall is armed.  Small
+// levels then sweep with the TMA kernel too, the one that can stall.
+static std::atomic<bool> g_stall_armed{false};
+
 // A device array.  alloc() keeps the current allocation when it is large
 // enough (rebuilt launch tables reuse their buffers).
 template <typename T>
@@ -980,6 +984,7 @@ struct View {
   cudaGraphExec_t x_loop = nullptr, x_once = nullptr;
   cudaGraphConditionalHandle cond = 0;
   long long launches_per_iter = 0;
+  bool graphs_armed = false;          // captured with g_stall_armed set
   void drop_graphs() {
     if (x_loop) cudaGraphExecDestroy(x_loop);
     if (g_loop) cudaGraphDestroy(g_loop);
@@ -1074,6 +1079,8 @@ static void prof_collect(mf3d_ctx *C) {
 
 // Levels with at most this many interior cells sweep with k_rbgs_small.
 constexpr long long kSmallLevelCells = 1ll << 19;
+// Levels of fewer cells keep that kernel, untuned.
+constexpr long long kTunedCells = 1ll << 17;
 
 // Red-black sweep segments of a set of blocks (k_rbgs).  A column is 32
 // lanes over q (ceil(nx/2) per row) by RB_RJ rows of one block.  Schedules:
@@ -1688,11 +1695,11 @@ static int build_view(mf3d_ctx *C, View &V, const std::vector<DomainStore *> &do
       L.n_rtma = (int)rm.size();
       if ((st = L.rtma.upload(rm, s))) return st;
     }
-    // level 1 always takes the pipelined sweep; MF3D_SMALL_LEVEL_CELLS overrides the limit
+    // MF3D_SMALL_LEVEL_CELLS overrides the limit
     long long small_limit = kSmallLevelCells;
     if (const char *e = std::getenv("MF3D_SMALL_LEVEL_CELLS")) small_limit = std::atoll(e);
     // under L_LSM every level sweeps with the plain-load kernel (per-cell coefficients)
-    L.small = C->prm.lsm || (g > 1 && L.cells_sub[SUB_A] <= small_limit);
+    L.small = C->prm.lsm || L.cells_sub[SUB_A] <= small_limit;
     for (int q = 0; q < 3; ++q) {
       std::vector<int> pre(1, 0);
       for (int b : li[q]) {
@@ -1917,7 +1924,7 @@ static void relax(mf3d_ctx *C, View &V, int g, int q, int it, bool from_zero, bo
       const bool skip_red = fz && red_done;  // the restriction formed the red half-sweep
       prof_begin(C, fz ? 0 : pk, 3 * half);
       const dim3 grid(L.n_sweep[q]), cta(RB_TX, RB_TY);
-      if (L.small) {
+      if (L.small && (C->prm.lsm || !g_stall_armed)) {
         const int g2 = grid_of(L.small_items[q], kTile);
         if (skip_red)
           ;
@@ -2195,7 +2202,11 @@ static int autotune_level(mf3d_ctx *C, View &V, int g, bool time_new) {
     const std::string ks = tune_key(C, L, "sweep", sizeof(T));
     int v;
     const char *forced = std::getenv("MF3D_SWEEP_SCHED");  // a fixed schedule (tuning comparisons)
-    if (forced) {
+    if (L.cells_sub[SUB_A] < kTunedCells && L.small) {
+      // the plain-load kernel: a level this small leaves most SMs idle in the
+      // TMA ring, whose fill alone takes longer (64 K cells on one block: 10
+      // us a half-sweep against 4)
+    } else if (forced) {
       if ((st = upload_sweeps(C, L, std::max(0, std::min(kSweepSchedules - 1, std::atoi(forced)))))) return st;
     } else if (g == 1) {
       // level 1 keeps the default: timed on its own (no outer kernels
@@ -2209,7 +2220,7 @@ static int autotune_level(mf3d_ctx *C, View &V, int g, bool time_new) {
       // candidates 0 .. kSweepSchedules-1: k_rbgs with that schedule;
       // kSweepSchedules: k_rbgs_small (levels of 64 K to 4 M cells)
       const long long cells = L.cells_sub[SUB_A];
-      const bool small_ok = g > 1 && cells >= (1LL << 16) && cells <= (1LL << 22);
+      const bool small_ok = g > 1 && cells >= kTunedCells && cells <= (1LL << 22);
       const int n = kSweepSchedules + (small_ok ? 1 : 0);
       const int Lc = C->coarse64 ? V.Lmax : V.Lmax + 1;
       const int ir = std::max(C->prm.irestr, 1), ip = C->prm.iproln;
@@ -2803,6 +2814,10 @@ static int solve_view(mf3d_ctx *C, View &V, const double *dt, const double *alfa
   long long iters_run = 0;
   if (maxcy > 0) {
     if (C->use_graph && C->prof_kind == 0) {
+      if (V.graphs_armed != g_stall_armed) {
+        V.drop_graphs();
+        V.graphs_armed = g_stall_armed;
+      }
       if ((st = build_graphs<T>(C, V)) && V.mid_on) {
         // a driver that does not capture the cooperative middle-level launch
         // into the loop graph: the launch path instead
@@ -3954,6 +3969,7 @@ int mf3d_test_stall_copy(int device, int bytes) {
   if (cudaSetDevice(device) != cudaSuccess) { mf3d::set_error("cudaSetDevice failed"); return MF3D_E_CUDA; }
   const cudaError_t e = cudaMemcpyToSymbol(mf3d::g_test_extra_tx, &bytes, sizeof(int));
   if (e != cudaSuccess) { mf3d::set_error(std::string("mf3d_test_stall_copy: ") + cudaGetErrorString(e)); return MF3D_E_CUDA; }
+  mf3d::g_stall_armed = bytes > 0;
   return MF3D_OK;
 }
 

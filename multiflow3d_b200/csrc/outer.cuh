@@ -858,12 +858,16 @@ constexpr int CV_TY = 4, CV_CR = OZ_RJ / CV_TY;  // 32 x CV_TY threads, CV_CR co
 // x / b for k_calvel_calmas_tma's march: on an EXACT axis the product with
 // the exact inverse; otherwise Markstein's correction of div_rcp without its
 // branch - `bad` records an x outside the range where the correction is the
-// IEEE quotient (zero, subnormal, huge, non-finite), and the tile then
-// divides again (cv_cells_divide).
+// IEEE quotient (-0, subnormal, huge, non-finite), and the tile then divides
+// again (cv_cells_divide).  +0 comes out as +0: a pressure that is still zero
+// (every solve from rest) and fluid at rest stay on the march.  Before, the
+// first calvel of a 256^3 solve divided every tile again: 890 us, now 205.
 template <bool EXACT>
 __device__ __forceinline__ double qdv(double x, double b, double rb, bool &bad) {
   if (EXACT) return x * rb;
-  bad |= !rcp_range(x);
+  const unsigned hi = (unsigned)__double2hiint(x);
+  // the exponent test of rcp_range on the doubled high word (the sign shifted out)
+  bad |= 2u * hi - (323u << 21) >= (1401u << 21) && (hi | (unsigned)__double2loint(x)) != 0u;
   const double q0 = x * rb;
   const double q1 = fma(fma(-b, q0, x), rb, q0);
   return fma(fma(-b, q1, x), rb, q1);
