@@ -96,8 +96,15 @@ __device__ __forceinline__ void sweep_cell(const BlkLev &B, const Coef<T> &cf, T
   M[base + h] = ((R[base + h] - (aw * w + ae * e + as * so + an * no + ab * bo + at * to)) / ap);
 }
 
+// The phases below are functions of their own, one copy of each per value
+// type: inlined at every call the kernel outgrew the instruction cache.
+// Arrays are byte offsets into the kernel's dynamic shared memory.
 template <typename T>
-__device__ __forceinline__ void cc_sweep(const BlkLev &B, T *phi, const T *rhs, int colour) {
+__device__ __noinline__ void cc_sweep(const BlkLev *Bp, unsigned phi_at, unsigned rhs_at, int colour) {
+  extern __shared__ __align__(16) unsigned char cc_smem[];
+  const BlkLev B = *Bp;
+  T *phi = (T *)(cc_smem + phi_at);
+  const T *rhs = (const T *)(cc_smem + rhs_at);
   const int Q = (B.nx + 1) / 2;
   const int items = Q * B.ny * B.nz;
   const Coef<T> cf(B);
@@ -166,8 +173,12 @@ __device__ __forceinline__ void restrict_cell(const BlkLev &Fb, const Coef<TF> &
 // coarse phi := 0 on every cell, the interior coarse rhs from the 8
 // children's residuals, and the coarse from-zero red half-sweep - k_restrict.
 template <typename TF, typename TC>
-__device__ __forceinline__ void cc_restrict(const BlkLev &Fb, const TF *P, const TF *R, const BlkLev &Cb, TC *PC,
-                                            TC *RC) {
+__device__ __noinline__ void cc_restrict(const BlkLev *Fp, unsigned p_at, unsigned r_at, const BlkLev *Cp,
+                                         unsigned pc_at, unsigned rc_at) {
+  extern __shared__ __align__(16) unsigned char cc_smem[];
+  const BlkLev Fb = *Fp, Cb = *Cp;
+  const TF *P = (const TF *)(cc_smem + p_at), *R = (const TF *)(cc_smem + r_at);
+  TC *PC = (TC *)(cc_smem + pc_at), *RC = (TC *)(cc_smem + rc_at);
   const int GX = Cb.nx + 2, GY = Cb.ny + 2, GZ = Cb.nz + 2;
   const Coef<TF> cf(Fb);
   const Coef<TC> cc(Cb);
@@ -236,12 +247,42 @@ __device__ __forceinline__ void prolong_group(const BlkLev &Fb, TF *PF, const Bl
 // mgcorr + mgbound from the coarse level (Cb, PC) onto the fine one (Fb, PF):
 // one 2x2x2 fine group per thread - k_prolong.
 template <typename TF, typename TC>
-__device__ __forceinline__ void cc_prolong(const BlkLev &Fb, TF *PF, const BlkLev &Cb, const TC *PC) {
+__device__ __noinline__ void cc_prolong(const BlkLev *Fp, unsigned pf_at, const BlkLev *Cp, unsigned pc_at) {
+  extern __shared__ __align__(16) unsigned char cc_smem[];
+  const BlkLev Fb = *Fp, Cb = *Cp;
+  TF *PF = (TF *)(cc_smem + pf_at);
+  const TC *PC = (const TC *)(cc_smem + pc_at);
   const int GX = Cb.nx + 1, GY = Cb.ny + 1, GZ = Cb.nz + 1;
   const FastDiv fx((unsigned)GX), fy((unsigned)GY);
   for (int t = threadIdx.x; t < GX * GY * GZ; t += blockDim.x) {
     const int r = (int)fx.div((unsigned)t), K = (int)fy.div((unsigned)r);
     prolong_group<TF, TC>(Fb, PF, Cb, PC, t - r * GX, r - K * GY, K);
+  }
+  __syncthreads();
+}
+
+// The halo refresh of level l: every source read (through DSMEM) before any
+// destination is written.  off: byte offset of each rank's level arrays.
+__device__ __noinline__ void cc_halo(const CcArgs *a, int l, const long long *off, unsigned buf_at, bool f64) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) unsigned char cc_smem[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int b = (int)cluster.block_rank();
+  const CcHalo H = a->halo[l * a->nb + b];
+  double *buf = (double *)(cc_smem + buf_at);
+  unsigned char *mine = cc_smem + off[b * CC_MAX_LEVELS + l];
+  cluster.sync();  // every block's sweep is complete
+  for (int t = threadIdx.x; t < H.n; t += blockDim.x) {
+    const HaloCopy c = H.pairs[t];
+    unsigned char *src =
+        (unsigned char *)cluster.map_shared_rank((void *)(cc_smem + off[c.sblk * CC_MAX_LEVELS + l]), c.sblk);
+    buf[t] = f64 ? ((const double *)src)[c.soff] : (double)((const float *)src)[c.soff];
+  }
+  cluster.sync();  // every source is read
+  for (int t = threadIdx.x; t < H.n; t += blockDim.x) {
+    const HaloCopy c = H.pairs[t];
+    if (f64) ((double *)mine)[c.doff] = buf[t];
+    else ((float *)mine)[c.doff] = (float)buf[t];
   }
   __syncthreads();
 }
@@ -327,29 +368,17 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_coarse_cycle(const CcArgs a, 
     }
   }
   __syncthreads();
-  // the halo refresh of level l: every source read (through DSMEM) before
-  // any destination is written
-  auto halo = [&](int l) {
-    const CcHalo H = a.halo[l * a.nb + b];
-    const bool f64 = a.g0 + l >= a.lc || sizeof(TF) == 8;
-    cluster.sync();  // every block's sweep is complete
-    for (int t = threadIdx.x; t < H.n; t += blockDim.x) {
-      const HaloCopy c = H.pairs[t];
-      unsigned char *src = (unsigned char *)cluster.map_shared_rank((void *)phi_at(c.sblk, l), c.sblk);
-      buf[t] = f64 ? ((const double *)src)[c.soff] : (double)((const float *)src)[c.soff];
-    }
-    cluster.sync();  // every source is read
-    for (int t = threadIdx.x; t < H.n; t += blockDim.x) {
-      const HaloCopy c = H.pairs[t];
-      if (f64) ((double *)phi_at(b, l))[c.doff] = buf[t];
-      else ((float *)phi_at(b, l))[c.doff] = (float)buf[t];
-    }
-    __syncthreads();
+  const unsigned buf_at = (unsigned)((unsigned char *)buf - cc_smem);
+  // the halo refresh of level l
+  auto halo = [&](int l) { cc_halo(&a, l, &off[0][0], buf_at, a.g0 + l >= a.lc || sizeof(TF) == 8); };
+  auto po = [&](int l) { return (unsigned)off[b][l]; };  // phi, rhs of level l
+  auto ro = [&](int l) {
+    const int elem = a.g0 + l >= a.lc ? 8 : (int)sizeof(TF);
+    return (unsigned)(off[b][l] + cc_level_bytes(sdesc[l], elem));
   };
   auto sweep = [&](int l, int colour) {
-    const BlkLev B = desc(l);
-    if (a.g0 + l >= a.lc) cc_sweep<double>(B, (double *)phi_at(b, l), (const double *)rhs_at(l), colour);
-    else cc_sweep<TF>(B, (TF *)phi_at(b, l), (const TF *)rhs_at(l), colour);
+    if (sizeof(TF) == 8 || a.g0 + l >= a.lc) cc_sweep<double>(&sdesc[l], po(l), ro(l), colour);
+    else cc_sweep<TF>(&sdesc[l], po(l), ro(l), colour);
   };
   const int top = a.nlev - 1;
   // down: each level's first red half-sweep was formed by the restriction into it
@@ -367,22 +396,17 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_coarse_cycle(const CcArgs a, 
       }
       break;
     }
-    const BlkLev Fb = desc(l), Cb = desc(l + 1);
-    const bool f64 = a.g0 + l >= a.lc, c64 = a.g0 + l + 1 >= a.lc;
-    if (f64) cc_restrict<double, double>(Fb, (const double *)phi_at(b, l), (const double *)rhs_at(l), Cb,
-                                         (double *)phi_at(b, l + 1), (double *)rhs_at(l + 1));
-    else if (c64) cc_restrict<TF, double>(Fb, (const TF *)phi_at(b, l), (const TF *)rhs_at(l), Cb,
-                                          (double *)phi_at(b, l + 1), (double *)rhs_at(l + 1));
-    else cc_restrict<TF, TF>(Fb, (const TF *)phi_at(b, l), (const TF *)rhs_at(l), Cb, (TF *)phi_at(b, l + 1),
-                             (TF *)rhs_at(l + 1));
+    const bool f64 = sizeof(TF) == 8 || a.g0 + l >= a.lc, c64 = sizeof(TF) == 8 || a.g0 + l + 1 >= a.lc;
+    if (f64) cc_restrict<double, double>(&sdesc[l], po(l), ro(l), &sdesc[l + 1], po(l + 1), ro(l + 1));
+    else if (c64) cc_restrict<TF, double>(&sdesc[l], po(l), ro(l), &sdesc[l + 1], po(l + 1), ro(l + 1));
+    else cc_restrict<TF, TF>(&sdesc[l], po(l), ro(l), &sdesc[l + 1], po(l + 1), ro(l + 1));
   }
   // up
   for (int l = top - 1; l >= 0; --l) {
-    const BlkLev Fb = desc(l), Cb = desc(l + 1);
-    const bool f64 = a.g0 + l >= a.lc, c64 = a.g0 + l + 1 >= a.lc;
-    if (f64) cc_prolong<double, double>(Fb, (double *)phi_at(b, l), Cb, (const double *)phi_at(b, l + 1));
-    else if (c64) cc_prolong<TF, double>(Fb, (TF *)phi_at(b, l), Cb, (const double *)phi_at(b, l + 1));
-    else cc_prolong<TF, TF>(Fb, (TF *)phi_at(b, l), Cb, (const TF *)phi_at(b, l + 1));
+    const bool f64 = sizeof(TF) == 8 || a.g0 + l >= a.lc, c64 = sizeof(TF) == 8 || a.g0 + l + 1 >= a.lc;
+    if (f64) cc_prolong<double, double>(&sdesc[l], po(l), &sdesc[l + 1], po(l + 1));
+    else if (c64) cc_prolong<TF, double>(&sdesc[l], po(l), &sdesc[l + 1], po(l + 1));
+    else cc_prolong<TF, TF>(&sdesc[l], po(l), &sdesc[l + 1], po(l + 1));
     for (int itr = 0; itr < a.ip; ++itr) {
       sweep(l, 0);
       sweep(l, 1);
