@@ -27,6 +27,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cooperative_groups.h>
 #include <cuda.h>  // CUtensorMap (type only: the library does not link the driver)
 #include <cuda_runtime.h>
 
@@ -722,6 +723,222 @@ __global__ void __launch_bounds__(TD_THREADS) k_tdma_lines(const BlkLev *__restr
       if (cl > 1) cluster_sync_all();
       else __syncthreads();
     }
+  }
+}
+
+// The same relaxation for blocks whose slice of a diagonal, at most 32 lines
+// a CTA, fits shared memory twice, with 1-D coefficients (no L_LSM).  A
+// line's new neighbours lie on the diagonal before, its old ones on the next,
+// so while one warp (a lane per line) runs a diagonal's recurrences the
+// others store the diagonal before and stage the next: su, a, apr and the
+// old neighbours by cp.async, then t = su - c1*n1 and c3*n3.  The new values
+// stay in shared memory from diagonal to diagonal (the last line of a slice
+// goes to the next CTA's).  A diagonal then costs rhs' of its cells, formed
+// by all warps, the chain of five dependent FP64 operations a cell and one
+// cluster barrier; k_tdma_lines adds the staging's round trip and the stores.
+// One relaxation of 8 blocks of 64^3: 1.40 ms against 2.32 (3.7 and 6.1 us a
+// diagonal), 128^3: 4 V-cycles of the whole hierarchy 127 ms against 160.  With rhs'
+// formed by the recurrences' warp 1.56 ms; TW_CH = 4 1.48 ms.
+constexpr int TW_THREADS = 256, TW_CH = 8, TW_LINES = 32;
+// elements of shared memory (of T) for lmax lines of nmax cells
+__host__ __device__ inline long long tw_elems(int lmax, int nmax, int coefs) {
+  const long long ld = (nmax + 1) | 1;
+  return 11LL * lmax * ld + 4 * ld + 4 * lmax + coefs;
+}
+template <typename T>
+__global__ void __launch_bounds__(TW_THREADS) k_tdma_wave(const BlkLev *__restrict__ bl, const int *__restrict__ blocks,
+                                                         const int *__restrict__ act, int cl, int lmax, int nmax) {
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char td_smem[];
+  const BlkLev B = bl[blocks[blockIdx.x / cl]];
+  if (!act[B.dom]) return;  // every CTA of the cluster holds the same block
+  const int rank = blockIdx.x % cl, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ld = (nmax + 1) | 1;  // odd: the lanes of a recurrence hit distinct banks
+  const int sl = lmax * ld;
+  T *tt = (T *)td_smem;       // [2] su, then t, then c
+  T *x3 = tt + 2 * sl;        // [2] old neighbour 3, then c3*n3
+  T *rp = x3 + 2 * sl;        // [2] apr
+  T *aa = rp + 2 * sl;        // [2] a
+  T *x1 = aa + 2 * sl;        // old neighbour 1
+  T *ph = x1 + sl;            // [2] the diagonal's new values
+  T *wl = ph + 2 * sl;        // [2] the line before the slice's first (u-1): the CTA before's last, or the ghost
+  T *gv = wl + 2 * ld;        // [2] the ghost line v = 0
+  T *g0 = gv + 2 * ld;        // [2] ghosts before m = 1 and after m = n
+  T *g1 = g0 + 2 * lmax;
+  T *co = g1 + 2 * lmax;      // the block's coefficients: aw ae as an ab at
+  T *P = phi_of<T>(B);
+  const T *R = rhs_of<T>(B);
+  const T *TF = (const T *)B.tdf;
+  const long long fn = (long long)B.nx * B.ny * B.nz;
+  for (int e = threadIdx.x; e < 2 * (B.nx + B.ny + B.nz + 6); e += TW_THREADS) co[e] = ((const T *)B.coef)[e];
+  const T *aw = co, *ae = aw + B.nx + 2, *as = ae + B.nx + 2, *an = as + B.ny + 2, *ab = an + B.ny + 2,
+          *at = ab + B.nz + 2;
+  T *wl_next = nullptr;  // the next CTA's wl
+  if (cl > 1) {
+    namespace cg = cooperative_groups;
+    if (rank + 1 < cl) wl_next = cg::this_cluster().map_shared_rank(wl, rank + 1);
+  }
+  auto sync = [&] {
+    __syncthreads();
+    if (cl > 1) cluster_sync_all();
+  };
+  for (int dir = 0; dir < 3; ++dir) {
+    int nu, nv, n;
+    tdma_dims(B, dir, nu, nv, n);
+    const int per = (nu + cl - 1) / cl, ulo = rank * per + 1, uhi = min(nu, ulo + per - 1);
+    const T *lo = dir == 0 ? as : dir == 1 ? aw : ab;
+    const T *cu1 = dir == 0 ? ae : dir == 1 ? an : ae, *cu0 = dir == 0 ? aw : dir == 1 ? as : aw;  // towards u+1, u-1
+    const T *cv1 = dir == 2 ? an : at, *cv0 = dir == 2 ? as : ab;                                  // towards v+1, v-1
+    sync();  // the coefficients; the previous pass's values
+    // the new values of diagonal s, slots (s & 1), by warps w0.. of nw
+    auto store = [&](int s, int w0, int nw) {
+      const int u0 = max(ulo, s - nv), u1 = min(uhi, s - 1);
+      for (int u = u0 + w0; u <= u1; u += nw) {
+        const T *src = ph + (s & 1) * sl + (u - ulo) * ld;
+        for (int m = lane + 1; m <= n; m += 32) {
+          int i, j, k;
+          tdma_cell(dir, u, s - u, m, i, j, k);
+          P[cell_off(B, i, j, k)] = src[m - 1];
+        }
+      }
+    };
+    for (int s = 1; s <= nu + nv; ++s) {
+      const int b = s & 1;
+      // rhs' = ((t - c2*n2) - c3*n3) - c4*n4 of the diagonal, every warp
+      if (s > 1) {
+        const int u0 = max(ulo, s - nv), u1 = min(uhi, s - 1);
+        for (int u = u0 + warp; u <= u1; u += TW_THREADS / 32) {
+          const int v = s - u, g = u - ulo;
+          T *t = tt + b * sl + g * ld;
+          const T *p3 = x3 + b * sl + g * ld;
+          const T *prev = ph + (b ^ 1) * sl + g * ld;
+          const T *nu0 = g ? prev - ld : wl + (b ^ 1) * ld;       // (u-1, v)
+          const T *nv0 = v > 1 ? prev : gv + (b ^ 1) * ld;        // (u, v-1)
+          const T *n2 = dir == 2 ? nv0 : nu0, *n4 = dir == 2 ? nu0 : nv0;
+          const T c2 = dir == 2 ? cv0[v] : cu0[u], c4 = dir == 2 ? cu0[u] : cv0[v];
+          for (int m = lane; m < n; m += 32) t[m] = ((t[m] - c2 * n2[m]) - p3[m]) - c4 * n4[m];
+        }
+        __syncthreads();
+      }
+      if (warp == 0) {
+        const int u = ulo + lane, v = s - u;
+        if (s > 1 && u <= uhi && v >= 1 && v <= nv) {
+          T *t = tt + b * sl + lane * ld;
+          const T *ar = rp + b * sl + lane * ld, *av = aa + b * sl + lane * ld;
+          T *out = ph + b * sl + lane * ld;
+          // batches of TW_CH cells, the next one's operands loaded beside the
+          // chain (reads past the line stay inside the arrays)
+          T r[TW_CH], z[TW_CH], y[TW_CH];
+          auto get = [&](int m0) {
+#pragma unroll
+            for (int q = 0; q < TW_CH; ++q) {
+              const int m = m0 + q;
+              r[q] = t[m];
+              z[q] = ar[m];
+              y[q] = lo[m + 1];
+            }
+          };
+          const int nf = n / TW_CH * TW_CH;
+          get(0);
+          T c = g0[b * lmax + lane];
+          for (int m0 = 0; m0 < nf; m0 += TW_CH) {
+            T rr[TW_CH], zz[TW_CH], yy[TW_CH];
+#pragma unroll
+            for (int q = 0; q < TW_CH; ++q) { rr[q] = r[q]; zz[q] = z[q]; yy[q] = y[q]; }
+            get(m0 + TW_CH);
+#pragma unroll
+            for (int q = 0; q < TW_CH; ++q) {
+              c = (rr[q] - yy[q] * c) * zz[q];
+              t[m0 + q] = c;
+            }
+          }
+          for (int q = 0; q < n - nf; ++q) {
+            const int m = nf + q;
+            c = (t[m] - lo[m + 1] * c) * ar[m];
+            t[m] = c;
+          }
+          T pv = g1[b * lmax + lane];
+          for (int m = n; m > nf; --m) {
+            pv = (t[m - 1] - av[m - 1] * pv);
+            out[m - 1] = pv;
+          }
+          auto back = [&](int m1) {  // cells m1-1 down to m1-TW_CH
+#pragma unroll
+            for (int q = 0; q < TW_CH; ++q) { r[q] = t[m1 - 1 - q]; z[q] = av[m1 - 1 - q]; }
+          };
+          if (nf > 0) back(nf);
+          for (int m1 = nf; m1 > 0; m1 -= TW_CH) {
+            T rr[TW_CH], zz[TW_CH];
+#pragma unroll
+            for (int q = 0; q < TW_CH; ++q) { rr[q] = r[q]; zz[q] = z[q]; }
+            if (m1 > TW_CH) back(m1 - TW_CH);
+#pragma unroll
+            for (int q = 0; q < TW_CH; ++q) {
+              pv = (rr[q] - zz[q] * pv);
+              out[m1 - 1 - q] = pv;
+            }
+          }
+        }
+        // the slice's last line also goes to the next CTA
+        if (s > 1 && uhi < nu && ulo <= uhi && s - uhi >= 1 && s - uhi <= nv) {
+          __syncwarp();
+          const T *src = ph + b * sl + (uhi - ulo) * ld;
+          for (int m = lane; m < n; m += 32) wl_next[b * ld + m] = src[m];
+        }
+      } else {
+        constexpr int NW = TW_THREADS / 32 - 1;
+        if (s > 2) store(s - 1, warp - 1, NW);
+        // stage diagonal s + 1: each line by one warp
+        const int ns = s + 1, nb = ns & 1;
+        const int u0 = max(ulo, ns - nv), u1 = min(uhi, ns - 1);
+        for (int u = u0 + warp - 1; u <= u1; u += NW) {
+          const int v = ns - u;
+          const long long o = nb * sl + (u - ulo) * ld;
+          int i, j, k;
+          for (int m = lane + 1; m <= n; m += 32) {
+            tdma_cell(dir, u, v, m, i, j, k);
+            cp_async_elem(tt + o + m - 1, R + cell_off(B, i, j, k));
+            const long long fo = tdma_fidx(B, dir, u, v, m, 0);
+            cp_async_elem(aa + o + m - 1, TF + fo);
+            cp_async_elem(rp + o + m - 1, TF + fo + fn);
+            tdma_cell(dir, u + 1, v, m, i, j, k);
+            const T *pu = P + cell_off(B, i, j, k);
+            tdma_cell(dir, u, v + 1, m, i, j, k);
+            const T *pw = P + cell_off(B, i, j, k);
+            cp_async_elem(x1 + (u - ulo) * ld + m - 1, dir == 2 ? pw : pu);
+            cp_async_elem(x3 + o + m - 1, dir == 2 ? pu : pw);
+            // the ghost lines the diagonal's ends read, into slot (ns-1) & 1
+            if (u == 1) {
+              tdma_cell(dir, 0, v, m, i, j, k);
+              cp_async_elem(wl + (nb ^ 1) * ld + m - 1, P + cell_off(B, i, j, k));
+            }
+            if (v == 1) {
+              tdma_cell(dir, u, 0, m, i, j, k);
+              cp_async_elem(gv + (nb ^ 1) * ld + m - 1, P + cell_off(B, i, j, k));
+            }
+          }
+          if (lane == 0) {
+            tdma_cell(dir, u, v, 0, i, j, k);
+            cp_async_elem(g0 + nb * lmax + (u - ulo), P + cell_off(B, i, j, k));
+            tdma_cell(dir, u, v, n + 1, i, j, k);
+            cp_async_elem(g1 + nb * lmax + (u - ulo), P + cell_off(B, i, j, k));
+          }
+        }
+        cp_async_wait_all();
+        __syncwarp();
+        for (int u = u0 + warp - 1; u <= u1; u += NW) {
+          const int v = ns - u;
+          const long long o = nb * sl + (u - ulo) * ld;
+          const T c1 = dir == 2 ? cv1[v] : cu1[u], c3 = dir == 2 ? cu1[u] : cv1[v];
+          for (int m = lane; m < n; m += 32) {
+            tt[o + m] = tt[o + m] - c1 * x1[(u - ulo) * ld + m];
+            x3[o + m] = c3 * x3[o + m];
+          }
+        }
+      }
+      sync();
+    }
+    store(nu + nv, warp, TW_THREADS / 32);
   }
 }
 

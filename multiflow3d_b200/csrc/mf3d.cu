@@ -912,6 +912,8 @@ struct ViewLevel {
   int td_cl = 1, td_gmax = 1, td_nmax = 1, td_numax = 1, td_lines[3] = {0, 0, 0};
   int lx_cl = 1;                      // lexicographic relaxation (mg_itrsch 1): CTAs per block
   size_t td_smem = 0;
+  int td_wave = 0;                    // k_tdma_wave: lines a CTA holds (0: k_tdma_lines)
+  int td_coefs = 0;                   // a block's 1-D coefficients at most; 0: per cell (no k_tdma_wave)
   bool td_fp64 = true;                // the level relaxes in FP64
   // LMR (single-domain views): the level's halo program where refinements
   // meet on it (DomainStore::LmrLevel), and the blocks past their own last
@@ -1221,6 +1223,38 @@ static int plane_tiles(const mf3d_ctx *C, const std::vector<PlaneExt> &ext, std:
   return best;
 }
 
+// Line relaxation shape for cl CTAs per block: k_tdma_wave where a CTA's
+// slice of a diagonal is at most a warp's lanes and shared memory holds it
+// with the next one's staging (1-D coefficients only), else k_tdma_lines with
+// as many lines staged at a time as fit.
+constexpr size_t kTdSmem = 200 * 1024, kTwSmem = 220 * 1024;
+static void td_shape(ViewLevel &L, int cl) {
+  const size_t sz = L.td_fp64 ? 8 : 4;
+  const int per = (L.td_numax + cl - 1) / cl;
+  L.td_cl = cl;
+  L.td_wave = 0;
+  if (L.td_coefs && per <= TW_LINES) {
+    const size_t smem = (size_t)tw_elems(per, L.td_nmax, L.td_coefs) * sz;
+    if (smem <= kTwSmem) {
+      L.td_wave = per;
+      L.td_smem = smem;
+      return;
+    }
+  }
+  L.td_gmax = (int)std::max<size_t>(1, std::min<size_t>(per, kTdSmem / ((7 * (size_t)L.td_nmax + 9) * sz)));
+  L.td_smem = (7 * (size_t)L.td_gmax * (L.td_nmax + 1) + 2 * (size_t)L.td_gmax) * sz;
+}
+// One line relaxation of the listed blocks of subset q.
+template <typename T>
+static void tdma_relax(mf3d_ctx *C, View &V, ViewLevel &L, int q) {
+  if (L.td_wave)
+    launch_cl(k_tdma_wave<T>, L.n_list[q] * L.td_cl, TW_THREADS, L.td_smem, C->stream, L.td_cl, L.tab.p, L.list[q].p,
+              V.act.p, L.td_cl, L.td_wave, L.td_nmax);
+  else
+    launch_cl(k_tdma_lines<T>, L.n_list[q] * L.td_cl, TD_THREADS, L.td_smem, C->stream, L.td_cl, L.tab.p, L.list[q].p,
+              V.act.p, L.td_cl, L.td_gmax, L.td_nmax);
+}
+
 // Line relaxation (mg_itrsch 2) on level g: room for every listed block's
 // TDMA factors (six arrays of its cells, k_tdma_factor), pointed to from its
 // table entry, and the shape of k_tdma_lines.  A block whose diagonals hold
@@ -1251,18 +1285,18 @@ static int tdma_layout(mf3d_ctx *C, View &V, int g, std::vector<BlkLev> &tab) {
   if ((st = L.tdf.alloc(std::max<size_t>(bytes, 256)))) return st;
   for (int b = 0; b < nb; ++b)
     if (g <= V.blk[b]->ngrid) tab[b].tdf = L.tdf.p + off[b];
-  const size_t cap = 200 * 1024;
-  // the kernel's limits (the attributes are the kernel's, not the launch's)
-  void (*kern)(const BlkLev *, const int *, const int *, int, int, int) =
-      L.td_fp64 ? (void (*)(const BlkLev *, const int *, const int *, int, int, int))k_tdma_lines<double>
-                : (void (*)(const BlkLev *, const int *, const int *, int, int, int))k_tdma_lines<float>;
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
-  // shape for cl CTAs per block: lines staged at a time and shared memory
-  auto shape = [&](int cl, int &gmax, size_t &smem) {
-    const int per = (numax + cl - 1) / cl;
-    gmax = (int)std::max<size_t>(1, std::min<size_t>(per, cap / ((7 * (size_t)nmax + 9) * sz)));
-    smem = (7 * (size_t)gmax * (nmax + 1) + 2 * (size_t)gmax) * sz;
-  };
+  L.td_coefs = 0;
+  if (!C->prm.lsm)
+    for (int b = 0; b < nb; ++b)
+      if (g <= V.blk[b]->ngrid) L.td_coefs = std::max(L.td_coefs, 2 * (tab[b].nx + tab[b].ny + tab[b].nz + 6));
+  L.td_nmax = nmax;
+  L.td_numax = numax;
+  // the kernels' limits (the attributes are the kernel's, not the launch's)
+  typedef void (*Kern)(const BlkLev *, const int *, const int *, int, int, int);
+  const Kern lines = L.td_fp64 ? (Kern)k_tdma_lines<double> : (Kern)k_tdma_lines<float>;
+  const Kern wave = L.td_fp64 ? (Kern)k_tdma_wave<double> : (Kern)k_tdma_wave<float>;
+  CK(cudaFuncSetAttribute(lines, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTdSmem));
+  CK(cudaFuncSetAttribute(wave, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTwSmem));
   // Up to 8 CTAs per block (portable clusters); more (non-portable, up to
   // 16) only where the device holds a cluster for every block of the level
   // at once - 16 with too few resident measured slower (18.1 against 11.2 ms
@@ -1271,34 +1305,32 @@ static int tdma_layout(mf3d_ctx *C, View &V, int g, std::vector<BlkLev> &tab) {
   L.td_cl = numax >= 32 ? std::min(8, numax / 8) : 1;
   int nblk = 0;
   for (int b = 0; b < nb; ++b) nblk += g <= V.blk[b]->ngrid;
-  if (numax >= 128 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
-    for (int cl = std::min(16, numax / 8); cl > 8; --cl) {
-      int gm;
-      size_t sm;
-      shape(cl, gm, sm);
+  if (numax >= 128 &&
+      cudaFuncSetAttribute(lines, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+      cudaFuncSetAttribute(wave, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+    const int portable = L.td_cl;
+    for (int cl = std::min(16, numax / 8); cl >= 8; --cl) {
+      td_shape(L, cl > 8 ? cl : portable);
+      if (cl == 8) break;
       cudaLaunchAttribute at;
       at.id = cudaLaunchAttributeClusterDimension;
       at.val.clusterDim.x = (unsigned)cl;
       at.val.clusterDim.y = at.val.clusterDim.z = 1;
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)cl);
-      cfg.blockDim = dim3(TD_THREADS);
-      cfg.dynamicSmemBytes = sm;
+      cfg.blockDim = dim3(L.td_wave ? TW_THREADS : TD_THREADS);
+      cfg.dynamicSmemBytes = L.td_smem;
       cfg.attrs = &at;
       cfg.numAttrs = 1;
       int ncl = 0;
-      if (cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg) == cudaSuccess && ncl >= nblk) {
-        L.td_cl = cl;
+      if (cudaOccupancyMaxActiveClusters(&ncl, L.td_wave ? wave : lines, &cfg) == cudaSuccess && ncl >= nblk)
         break;
-      }
     }
     cudaGetLastError();  // a refused query leaves no error behind
   }
   if (const char *e = std::getenv("MF3D_TD_CLUSTER")) L.td_cl = std::max(1, std::min(16, std::atoi(e)));  // tuning
-  shape(L.td_cl, L.td_gmax, L.td_smem);
-  L.td_nmax = nmax;
-  L.td_numax = numax;
-  if (L.td_smem > cap) {
+  td_shape(L, L.td_cl);
+  if ((7 * (size_t)(nmax + 1) + 2) * sz > kTdSmem) {
     set_error("line relaxation: a line of " + std::to_string(nmax) + " cells does not fit in shared memory");
     return MF3D_E_UNSUPPORTED;
   }
@@ -1960,8 +1992,7 @@ static void relax(mf3d_ctx *C, View &V, int g, int q, int it, bool from_zero, bo
       // three passes, each reading rhs and phi and writing phi once
       const int pk = (g == 1 && q == SUB_A) ? MF3D_PROF_SMOOTH_L1 : 0;
       prof_begin(C, pk, 9.0 * (double)L.cells_sub[q] * sizeof(T));
-      launch_cl(k_tdma_lines<T>, L.n_list[q] * L.td_cl, TD_THREADS, L.td_smem, C->stream, L.td_cl, L.tab.p,
-                L.list[q].p, V.act.p, L.td_cl, L.td_gmax, L.td_nmax);
+      tdma_relax<T>(C, V, L, q);
       prof_end(C, pk);
       ++C->launches;
     }
@@ -2180,15 +2211,6 @@ static int upload_sweeps(mf3d_ctx *C, ViewLevel &L, int sched, int only_q = -1) 
   L.sched = sched;
   return MF3D_OK;
 }
-// line relaxation shape for cl CTAs per block (as tdma_layout's)
-static void td_shape(ViewLevel &L, int cl) {
-  const size_t sz = L.td_fp64 ? 8 : 4, cap = 200 * 1024;
-  const int per = (L.td_numax + cl - 1) / cl;
-  L.td_gmax = (int)std::max<size_t>(1, std::min<size_t>(per, cap / ((7 * (size_t)L.td_nmax + 9) * sz)));
-  L.td_smem = (7 * (size_t)L.td_gmax * (L.td_nmax + 1) + 2 * (size_t)L.td_gmax) * sz;
-  L.td_cl = cl;
-}
-
 template <typename T>
 static int autotune_level(mf3d_ctx *C, View &V, int g, bool time_new) {
   ViewLevel &L = V.lv[g];
@@ -2268,8 +2290,7 @@ static int autotune_level(mf3d_ctx *C, View &V, int g, bool time_new) {
                C, (int)cls.size(), 0, [&](int c) { set_cl(cls[c]); return (int)MF3D_OK; },
                [&] {
                  if (sch == 2)
-                   launch_cl(k_tdma_lines<T>, L.n_list[SUB_A] * L.td_cl, TD_THREADS, L.td_smem, s, L.td_cl, L.tab.p,
-                             L.list[SUB_A].p, V.act.p, L.td_cl, L.td_gmax, L.td_nmax);
+                   tdma_relax<T>(C, V, L, SUB_A);
                  else
                    launch_cl(k_lexgs<T>, L.n_list[SUB_A] * L.lx_cl, 1024, 0, s, L.lx_cl, L.tab.p, L.list[SUB_A].p,
                              V.act.p, L.lx_cl);
@@ -2916,7 +2937,7 @@ static int preload_vcycle_kernels() {
       (const void *)k_rbgs_small<double, false>, (const void *)k_rbgs<double, true>,
       (const void *)k_rbgs<double, false>, (const void *)k_lexgs<T>, (const void *)k_lexgs<double>,
       (const void *)k_tdma_factor<T>, (const void *)k_tdma_factor<double>, (const void *)k_tdma_lines<T>,
-      (const void *)k_tdma_lines<double>, (const void *)k_restrict<T, T>, (const void *)k_restrict<T, double>,
+      (const void *)k_tdma_lines<double>, (const void *)k_tdma_wave<T>, (const void *)k_tdma_wave<double>, (const void *)k_restrict<T, T>, (const void *)k_restrict<T, double>,
       (const void *)k_restrict_tma<T, T>, (const void *)k_restrict_tma<T, double>, (const void *)k_prolong<T, T>,
       (const void *)k_prolong<T, double>, (const void *)k_halo_stage<T>, (const void *)k_halo_apply<T>,
       (const void *)k_halo_stage<double>, (const void *)k_halo_apply<double>, (const void *)k_zero_ghosts<T>,
