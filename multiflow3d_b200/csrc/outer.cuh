@@ -946,6 +946,7 @@ __global__ void __launch_bounds__(OZ_TX *CV_TY, CV_MINB) k_calvel_calmas_tma(con
   __shared__ __align__(128) unsigned char sbuf[CV_NS * S::STAGE];
   __shared__ __align__(8) uint64_t bar[CV_NS];
   __shared__ double red[CV_TY];
+  __shared__ double szm[OZ_KCH][4];  // the run's planes: df, RN(1/df), h, RN(1/h) of z
   const Tile t = tiles[blockIdx.x];
   if (!act[fl[t.blk].dom]) return;
   const BlkFld F = fl[t.blk];  // by value: read once, never reloaded after the stores below
@@ -1024,8 +1025,15 @@ __global__ void __launch_bounds__(OZ_TX *CV_TY, CV_MINB) k_calvel_calmas_tma(con
   if (!UY)
 #pragma unroll
     for (int m = 0; m < CV_CR; ++m) fast = fast && rhy[m] != 0.0 && rdyn[m] != 0.0 && rdys[m] != 0.0;
-  if (!UZ)
-    for (int kk = k0; kk <= k1; ++kk) fast = fast && F.rdf[2][kk] != 0.0 && F.rh[2][kk] != 0.0;
+  if (tid <= k1 - k0) {
+    const int kk = k0 + tid;
+    const double d = F.df[2][kk], h = F.h[2][kk], rd = UZ ? iz : F.rdf[2][kk], rh = UZ ? iz : F.rh[2][kk];
+    szm[tid][0] = d;
+    szm[tid][1] = rd;
+    szm[tid][2] = h;
+    szm[tid][3] = rh;
+    fast = fast && rd != 0.0 && rh != 0.0;
+  }
   double vmax = 0.0;
   bool bad = !__syncthreads_and(fast);
   if (!bad) {
@@ -1044,8 +1052,8 @@ __global__ void __launch_bounds__(OZ_TX *CV_TY, CV_MINB) k_calvel_calmas_tma(con
     const double *P = (const double *)b, *U = (const double *)(b + S::PB);
     const double *Vv = (const double *)(b + S::PB + S::UB), *Wv = (const double *)(b + S::PB + S::UB + S::VB);
     const double *PN = (const double *)(sbuf + stage(k + 1) * S::STAGE);
-    const double dzk = F.df[2][k], hzk = F.h[2][k];
-    const double rdzk = UZ ? iz : F.rdf[2][k], rhzk = UZ ? iz : F.rh[2][k];
+    const double *zm = szm[k - k0];
+    const double dzk = UZ ? 0.0 : zm[0], hzk = zm[2], rdzk = UZ ? iz : zm[1], rhzk = UZ ? iz : zm[3];
     const bool top = k == nz && twall;
     double vprev = 0.0;
 #pragma unroll
