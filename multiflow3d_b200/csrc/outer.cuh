@@ -971,8 +971,7 @@ __global__ void __launch_bounds__(OZ_TX *CV_TY, CV_MINB) k_calvel_calmas_tma(con
   int jc[CV_CR];
   bool in[CV_CR];
   double hy[CV_CR], dyn[CV_CR], dys[CV_CR], wb[CV_CR], rhy[CV_CR], rdyn[CV_CR], rdys[CV_CR];
-  long long l1off[CV_CR];  // level-1 element of (i, j, 0) without the colour term
-  int c0[CV_CR];           // colour of (i, j, 0)
+  T *rp[CV_CR];            // level-1 rhs of the thread's cell on the march's plane
   const long long ps1 = (long long)(F.L1.ny + 2) * F.L1.hp, sz = (long long)F.ti * F.tj;
   const int k0 = t.k0, k1 = min(t.k0 + kch - 1, nz);
 #pragma unroll
@@ -986,8 +985,7 @@ __global__ void __launch_bounds__(OZ_TX *CV_TY, CV_MINB) k_calvel_calmas_tma(con
     rhy[m] = UY ? iy : F.rh[1][jc[m]];
     rdyn[m] = UY ? iy : F.rdf[1][jc[m]];
     rdys[m] = UY ? iy : F.rdf[1][jc[m] - 1];
-    l1off[m] = (long long)j * F.L1.hp + (i >> 1);
-    c0[m] = (i + j + 1) & 1;
+    rp[m] = rhs1 + (((i + j + k0 + 1) & 1) ? F.L1.cstr : 0) + k0 * ps1 + (long long)j * F.L1.hp + (i >> 1);
     // w on the face below plane k0, carried up the march (plain loads)
     const long long c = fidx(F, ic, jc[m], k0);
     if (k0 == 1) {
@@ -1034,6 +1032,9 @@ __global__ void __launch_bounds__(OZ_TX *CV_TY, CV_MINB) k_calvel_calmas_tma(con
     szm[tid][3] = rh;
     fast = fast && rd != 0.0 && rh != 0.0;
   }
+  // a plane up is the other colour: ps1 + cstr from colour 0, ps1 - cstr from 1
+  const long long up0 = ps1 + F.L1.cstr, up1 = ps1 - F.L1.cstr;
+  bool odd = (i + t.j0 + CV_CR * ty + k0 + 1) & 1;  // colour of row 0's cell
   double vmax = 0.0;
   bool bad = !__syncthreads_and(fast);
   if (!bad) {
@@ -1096,13 +1097,15 @@ __global__ void __launch_bounds__(OZ_TX *CV_TY, CV_MINB) k_calvel_calmas_tma(con
       const double su = dtinv != 0.0 ? fact * dtinv : qdv<false>(fact, dt, rdt, cb);
       bad |= cb && in[m];
       if (ok && in[m]) {
-        rhs1[((c0[m] ^ (k & 1)) ? F.L1.cstr : 0) + k * ps1 + l1off[m]] = (T)su;
+        *rp[m] = (T)su;
         if (SU) SU[fidx(F, i, jc[m], k)] = su;
         double f1 = fabs(fact * hx * hy[m] * hzk);
         if (!(f1 == f1)) f1 = __longlong_as_double(0x7ff0000000000000LL);  // NaN -> +Inf (flagged)
         vmax = vmax > f1 ? vmax : f1;
       }
+      rp[m] += odd == (m & 1) ? up0 : up1;  // row m's colour is odd ^ (m & 1)
     }
+    odd = !odd;
     if (__syncthreads_or(!ok)) return;  // plane k's slot is refilled next iteration
   }
   }
