@@ -527,7 +527,10 @@ static int build_block(BlockStore &S, const mf3d_block_desc &d, int ngrid, int e
     F.bcst = S.bcst.p;
     S.bytes += S.bcst.n * sizeof(double);
   }
-  for (int a = 0; a < 3; ++a) F.pinv[a] = ext[a] ? 0.0 : pow2_inverse(hh[a]);
+  for (int a = 0; a < 3; ++a) {
+    F.uni[a] = ext[a] ? 0 : 1;
+    F.pinv[a] = ext[a] ? 0.0 : pow2_inverse(hh[a]);
+  }
   return MF3D_OK;
 }
 
@@ -2441,16 +2444,29 @@ static void calvel_calmas(mf3d_ctx *C, View &V, const int *act, unsigned long lo
   } else if (V.fields_tma) {
     // axes that are uniform with a power-of-two spacing in every block
     int mask = 7;
+    bool uni = true;  // no block has a stretched axis
     for (const auto &F : V.hf)
-      for (int a = 0; a < 3; ++a)
+      for (int a = 0; a < 3; ++a) {
         if (F.pinv[a] == 0.0) mask &= ~(1 << a);
+        uni = uni && F.uni[a];
+      }
     const dim3 grid(V.n_zint), cta(OZ_TX, CV_TY);
-#define MF3D_CV(M)                                                                                              \
-  case M:                                                                                                        \
-    launch(k_calvel_calmas_tma<T, M>, grid, cta, 0, C->stream, V.df.p, V.t_zint.p, V.ds.p, act, slot, write_su, OZ_KCH, \
-                                                           V.err.p);                                             \
-    break;
-    switch (mask) { MF3D_CV(0) MF3D_CV(1) MF3D_CV(2) MF3D_CV(3) MF3D_CV(4) MF3D_CV(5) MF3D_CV(6) MF3D_CV(7) }
+#define MF3D_CV(M, U)                                                                                                  \
+  launch(k_calvel_calmas_tma<T, M, U>, grid, cta, 0, C->stream, V.df.p, V.t_zint.p, V.ds.p, act, slot, write_su, OZ_KCH, \
+         V.err.p)
+    switch (mask) {
+      case 0:
+        if (uni) MF3D_CV(0, true);
+        else MF3D_CV(0, false);
+        break;
+      case 1: MF3D_CV(1, false); break;
+      case 2: MF3D_CV(2, false); break;
+      case 3: MF3D_CV(3, false); break;
+      case 4: MF3D_CV(4, false); break;
+      case 5: MF3D_CV(5, false); break;
+      case 6: MF3D_CV(6, false); break;
+      case 7: MF3D_CV(7, true); break;
+    }
 #undef MF3D_CV
   } else
     launch(k_calvel_calmas<T>, V.n_zint, dim3(OZ_TX, OZ_RJ), 0, C->stream, V.df.p, V.t_zint.p, V.ds.p, act, slot,
