@@ -120,7 +120,7 @@ struct Tile {
 // per CTA); planes per CTA chosen per level
 constexpr int RB_TX = 32, RB_TY = 4, RB_CR = 4, RB_RJ = RB_TY * RB_CR;
 constexpr int RW_TX = 32, RW_RJ = 8, RW_KCH = 8;    // row tiles, RW_KCH planes per CTA
-constexpr int OZ_TX = 32, OZ_RJ = 8, OZ_KCH = 16;   // outer calvel/calmas z-march
+constexpr int OZ_TX = 32, OZ_RJ = 8, OZ_KCH = 16;   // outer calvel/calmas z-march (OZ_KCH planes per CTA at most)
 
 // ---------------------------------------------------------------------------
 // TMA and mbarrier primitives (inline PTX, sm_90+ forms; built for sm_100a).

@@ -949,6 +949,7 @@ struct View {
   // (BlkFld::pface 1, 2); a face without a neighbour
   bool bc_alone[3] = {false, false, false}, bc_partner[3] = {false, false, false}, bc_wall[3] = {false, false, false};
   int n_pairs = 0, pairs_kch = 1;
+  int zkch = OZ_KCH;                  // planes per CTA of t_zint
   int n_int = 0, n_zint = 0, n_l1cells = 0, n_faces = 0, n_planes = 0, n_vfaces = 0;
   // field exchanges as copy maps (a view over one domain that has them):
   // exchange(1..3) of u, v, w and exchange(4) + pbound of p
@@ -1817,7 +1818,6 @@ static int build_view(mf3d_ctx *C, View &V, const std::vector<DomainStore *> &do
     const mf3d_block_desc &x = S.d;
     add_tiles_2d(t1, b, Box{1, x.nx, 1, x.ny, 1, x.nz}, RW_TX, RW_RJ, RW_KCH);
     add_tiles_2d(t2, b, Box{0, x.nx + 1, 0, x.ny + 1, 0, x.nz + 1}, RW_TX, RW_RJ, RW_KCH);
-    add_tiles_2d(t5, b, Box{1, x.nx, 1, x.ny, 1, x.nz}, OZ_TX, OZ_RJ, OZ_KCH);
     it_faces.push_back(2 * ((long long)x.ny * x.nz + (long long)x.nx * x.nz + (long long)x.nx * x.ny));
     it_planes.push_back((long long)x.ny * x.nz + (long long)x.nx * x.nz + (long long)x.nx * x.ny);
     it_vfaces.push_back((long long)(C->prm.pl_ex + 1) * it_faces.back());
@@ -1845,6 +1845,26 @@ static int build_view(mf3d_ctx *C, View &V, const std::vector<DomainStore *> &do
     V.pairs_kch = plane_tiles(C, pe, tp);
     V.n_pairs = (int)tp.size();
     if ((st = V.t_pairs.upload(tp, s))) return st;
+  }
+  // planes per CTA of calvel/calmas: the march of a CTA is serial, so few
+  // tiles take short runs (16 tiles of 64x32x32 cells: 33 us at 16 planes);
+  // 3 stands for a run's own start
+  {
+    const long long resident = (long long)C->nsm * (C->prm.lsm ? 4 : 6);
+    double best_cost = 1e300;
+    for (int kc : {2, 4, 8, OZ_KCH}) {
+      long long n = 0;
+      for (int b = 0; b < nb; ++b) {
+        const mf3d_block_desc &x = V.blk[b]->d;
+        n += (long long)((x.nx + OZ_TX - 1) / OZ_TX) * ((x.ny + OZ_RJ - 1) / OZ_RJ) * ((x.nz + kc - 1) / kc);
+      }
+      const double cost = (double)((n + resident - 1) / resident) * (kc + 3);
+      if (cost <= best_cost) { best_cost = cost; V.zkch = kc; }
+    }
+    for (int b = 0; b < nb; ++b) {
+      const mf3d_block_desc &x = V.blk[b]->d;
+      add_tiles_2d(t5, b, Box{1, x.nx, 1, x.ny, 1, x.nz}, OZ_TX, OZ_RJ, V.zkch);
+    }
   }
   auto t3 = make_tiles(it_faces), t4 = make_tiles(it_planes), t6 = make_tiles(it_vfaces);
   V.n_int = (int)t1.size(); V.n_l1cells = (int)t2.size(); V.n_faces = (int)t3.size();
@@ -2440,7 +2460,7 @@ static void calvel_calmas(mf3d_ctx *C, View &V, const int *act, unsigned long lo
   }
   if (C->prm.lsm) {
     launch(k_calvel_calmas_lsm, V.n_zint, dim3(OZ_TX, OZ_RJ), 0, C->stream, V.df.p, V.t_zint.p, V.ds.p, act, slot,
-           write_su);
+           write_su, V.zkch);
   } else if (V.fields_tma) {
     // axes that are uniform with a power-of-two spacing in every block
     int mask = 7;
@@ -2452,7 +2472,7 @@ static void calvel_calmas(mf3d_ctx *C, View &V, const int *act, unsigned long lo
       }
     const dim3 grid(V.n_zint), cta(OZ_TX, CV_TY);
 #define MF3D_CV(M, U)                                                                                                  \
-  launch(k_calvel_calmas_tma<T, M, U>, grid, cta, 0, C->stream, V.df.p, V.t_zint.p, V.ds.p, act, slot, write_su, OZ_KCH, \
+  launch(k_calvel_calmas_tma<T, M, U>, grid, cta, 0, C->stream, V.df.p, V.t_zint.p, V.ds.p, act, slot, write_su, V.zkch, \
          V.err.p)
     switch (mask) {
       case 0:
@@ -2470,7 +2490,7 @@ static void calvel_calmas(mf3d_ctx *C, View &V, const int *act, unsigned long lo
 #undef MF3D_CV
   } else
     launch(k_calvel_calmas<T>, V.n_zint, dim3(OZ_TX, OZ_RJ), 0, C->stream, V.df.p, V.t_zint.p, V.ds.p, act, slot,
-                                                                      write_su);
+                                                                      write_su, V.zkch);
 }
 
 // One outer iteration of newsolv_mg (newsolv_mg.for:25-58) for every active

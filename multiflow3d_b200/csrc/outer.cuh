@@ -645,7 +645,7 @@ __global__ void __launch_bounds__(OZ_TX *OZ_RJ) k_calvel_calmas(const BlkFld *__
                                                                const DomState *__restrict__ ds,
                                                                const int *__restrict__ act,
                                                                unsigned long long *__restrict__ rmax_slot,
-                                                               int write_su) {
+                                                               int write_su, int kch) {
   pdl_wait();
   __shared__ double red[OZ_RJ];
   const Tile t = tiles[blockIdx.x];
@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(OZ_TX *OZ_RJ) k_calvel_calmas(const BlkFld *__
   const double dyn = F.df[1][jc], dys = F.df[1][jc - 1];
   const bool ewall = F.wall[1], nwall = F.wall[3], twall = F.wall[5];
   const bool wwall = F.wall[0], swall = F.wall[2], bwall = F.wall[4];
-  const int k1 = min(t.k0 + OZ_KCH - 1, nz);
+  const int k1 = min(t.k0 + kch - 1, nz);
   double vmax = 0.0;
   // w on the face below plane k0, carried up the march
   double wb;
@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(OZ_TX *OZ_RJ) k_calvel_calmas_lsm(const BlkFld
                                                                    const DomState *__restrict__ ds,
                                                                    const int *__restrict__ act,
                                                                    unsigned long long *__restrict__ rmax_slot,
-                                                                   int write_su) {
+                                                                   int write_su, int kch) {
   pdl_wait();
   __shared__ double red[OZ_RJ];
   const Tile t = tiles[blockIdx.x];
@@ -774,7 +774,7 @@ __global__ void __launch_bounds__(OZ_TX *OZ_RJ) k_calvel_calmas_lsm(const BlkFld
   const double dx = F.df[0][ic], dy = F.df[1][jc];
   const bool ewall = F.wall[1], nwall = F.wall[3], twall = F.wall[5];
   const bool wwall = F.wall[0], swall = F.wall[2], bwall = F.wall[4];
-  const int k1 = min(t.k0 + OZ_KCH - 1, nz);
+  const int k1 = min(t.k0 + kch - 1, nz);
   double vmax = 0.0;
   double wcarry = 0.0;  // the top face of the previous plane: this plane's bottom face
   for (int k = t.k0; k <= k1; ++k) {
