@@ -289,13 +289,11 @@ __device__ __noinline__ void cc_halo(const CcArgs *a, int l, const long long *of
 
 template <typename TF>
 __global__ void __launch_bounds__(CC_THREADS, 1) k_coarse_cycle(const CcArgs a, const int *__restrict__ act) {
-  pdl_wait();
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char cc_smem[];
   __shared__ long long off[CC_MAX_BLOCKS][CC_MAX_LEVELS];  // byte offset of each rank's level arrays
   __shared__ BlkLev sdesc[CC_MAX_LEVELS];  // this block's levels, coefficients in shared memory
-  if (!act[a.dom]) return;  // the whole cluster is one domain: uniform
   const int b = (int)cluster.block_rank();
   if (threadIdx.x < a.nlev) sdesc[threadIdx.x] = a.tab[threadIdx.x][a.blk0 + b];
   if (threadIdx.x < a.nb) {
@@ -343,6 +341,8 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_coarse_cycle(const CcArgs a, 
     const int elem = a.g0 + l >= a.lc ? 8 : (int)sizeof(TF);
     return cc_smem + off[b][l] + cc_level_bytes(desc(l), elem);
   };
+  pdl_wait();
+  if (!act[a.dom]) return;  // the whole cluster is one domain: uniform
   // level g0 from global memory (rhs and phi, ghost shell included)
   {
     const BlkLev B = desc(0);

@@ -96,14 +96,24 @@ __device__ __forceinline__ void cell_coefs(const BlkLev &B, const Coef<T> &cf, i
 // with programmatic stream serialisation, so a kernel's CTAs may be resident
 // before the kernel it depends on has finished: they are placed as that
 // kernel's CTAs retire, instead of after a full drain and a launch gap.
-// Every kernel therefore begins with this wait, which returns once all
-// prerequisite grids have completed and their memory operations are
-// visible; nothing is read or written before it.  Without a programmatic
-// predecessor it returns at once.  No kernel signals its dependents early
-// (griddepcontrol.launch_dependents): the next grid launches as this one's
-// CTAs exit.  Signalling right after the wait measured slower (11.0 against
-// 11.4 solves/s), the waiting CTAs taking issue slots from the last wave.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Every kernel therefore waits first (pdl_wait), which returns once all
+// prerequisite grids have completed and their memory operations are visible;
+// before it a kernel reads only tables that no kernel of a solve writes (work
+// lists, descriptors, 1-D coefficients).  Without a programmatic predecessor
+// it returns at once.  A grid of one wave then signals its dependents
+// (griddepcontrol.launch_dependents): the next grid is placed and reads its
+// tables while this one works, which hides most of a small level's launch.
+// Larger grids signal by exiting: signalling right after the wait measured
+// slower there (11.0 against 11.4 solves/s at 256^3), the waiting CTAs
+// taking issue slots from the last wave.
+// 64x32x32 channel 1555 -> 1370 us a solve, 128^3 variable density 27.2 ->
+// 25.5 ms, 256^3 81.5 -> 80.7 ms.
+constexpr unsigned kPdlCtas = 592;
+__device__ __forceinline__ bool pdl_one_wave() { return gridDim.x * gridDim.y <= kPdlCtas; }
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (pdl_one_wave()) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // A CTA's work: block position and the origin of its tile.  2-D tiles:
 // threadIdx.x runs along i (or the compact index h), threadIdx.y along j;
@@ -408,17 +418,15 @@ template <typename T, bool FROM_ZERO>
 __global__ void __launch_bounds__(kTile) k_rbgs_small(const BlkLev *__restrict__ bl, const int *__restrict__ pre,
                                                       const int *__restrict__ blocks, int nb,
                                                       const int *__restrict__ act, int colour) {
-  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= pre[nb]) return;
+  if (t >= pre[nb]) return pdl_wait();
   int lo = 0, hi = nb - 1;  // last list entry whose first item <= t
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (pre[mid] <= t) lo = mid;
     else hi = mid - 1;
   }
-  const BlkLev &B = bl[blocks[lo]];
-  if (!act[B.dom]) return;
+  const BlkLev B = bl[blocks[lo]];
   const int Q = (B.nx + 1) / 2;
   int r = t - pre[lo];
   const int q = r % Q;
@@ -426,13 +434,18 @@ __global__ void __launch_bounds__(kTile) k_rbgs_small(const BlkLev *__restrict__
   const int j = r % B.ny + 1, k = r / B.ny + 1;
   const int s = (colour + j + k + 1) & 1;
   const int i = 2 * q + 2 - s;
-  if (i > B.nx) return;
   const Coef<T> cf(B);
   const long long rs = (long long)(B.ny + 2) * B.hp, base = (long long)k * rs + (long long)j * B.hp;
   const int h = q + 1 - s;
   const T *O = phi_of<T>(B) + (1 - colour) * B.cstr;
   T *M = phi_of<T>(B) + colour * B.cstr;
   const T *R = rhs_of<T>(B) + colour * B.cstr;
+  T aw, ae, as, an, ab, at;
+  const bool early = !B.cc && pdl_one_wave();  // (per-cell coefficients: a kernel of the solve formed them)
+  if (early) cell_coefs(B, cf, min(i, B.nx), j, k, aw, ae, as, an, ab, at);
+  pdl_wait();
+  if (!act[B.dom] || i > B.nx) return;
+  if (!early) cell_coefs(B, cf, i, j, k, aw, ae, as, an, ab, at);
   T w = (T)0, e = (T)0, so = (T)0, no = (T)0, bo = (T)0, to = (T)0;
   if (!FROM_ZERO) {
     w = O[base + q];
@@ -442,8 +455,6 @@ __global__ void __launch_bounds__(kTile) k_rbgs_small(const BlkLev *__restrict__
     bo = O[base - rs + h];
     to = O[base + rs + h];
   }
-  T aw, ae, as, an, ab, at;
-  cell_coefs(B, cf, i, j, k, aw, ae, as, an, ab, at);
   const T ap = (T)-1.0 * (aw + ae + as + an + ab + at);
   M[base + h] = ((R[base + h] - (aw * w + ae * e + as * so + an * no + ab * bo + at * to)) / ap);
 }
@@ -1318,26 +1329,42 @@ __device__ __forceinline__ int halo_segment(const HaloSeg *__restrict__ seg, int
 template <typename T>
 __global__ void k_halo_stage(const BlkLev *__restrict__ bl, const HaloSeg *__restrict__ seg, int nseg,
                              long long nstaged, const int *__restrict__ act, T *__restrict__ buf) {
-  pdl_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nstaged) return;
+  if (t >= nstaged) return pdl_wait();
   const HaloSeg &S = seg[halo_segment<true>(seg, nseg, t)];
-  if (!act[S.dom]) return;
+  const bool early = pdl_one_wave();
+  if (!early) {
+    pdl_wait();
+    if (!act[S.dom]) return;
+  }
   const HaloCopy c = S.pairs[t - S.sstart];
-  buf[t] = phi_of<T>(bl[S.blk_base + c.sblk])[c.soff];
+  const T *src = phi_of<T>(bl[S.blk_base + c.sblk]) + c.soff;
+  if (early) {
+    pdl_wait();
+    if (!act[S.dom]) return;
+  }
+  buf[t] = *src;
 }
 template <typename T>
 __global__ void k_halo_apply(const BlkLev *__restrict__ bl, const HaloSeg *__restrict__ seg, int nseg, long long n,
                              const int *__restrict__ act, const T *__restrict__ buf) {
-  pdl_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
+  if (t >= n) return pdl_wait();
   const HaloSeg &S = seg[halo_segment<false>(seg, nseg, t)];
-  if (!act[S.dom]) return;
+  const bool early = pdl_one_wave();  // larger grids look at act before they read pairs
+  if (!early) {
+    pdl_wait();
+    if (!act[S.dom]) return;
+  }
   const long long u = t - S.start;
   const HaloCopy c = S.pairs[u];
-  const T v = u < S.nstaged ? buf[S.sstart + u] : phi_of<T>(bl[S.blk_base + c.sblk])[c.soff];
-  phi_of<T>(bl[S.blk_base + c.dblk])[c.doff] = v;
+  const T *src = u < S.nstaged ? buf + S.sstart + u : phi_of<T>(bl[S.blk_base + c.sblk]) + c.soff;
+  T *dst = phi_of<T>(bl[S.blk_base + c.dblk]) + c.doff;
+  if (early) {
+    pdl_wait();
+    if (!act[S.dom]) return;
+  }
+  *dst = *src;
 }
 
 // Zero the ghost shell of a set of blocks (pp = 0 before a V-cycle): one
