@@ -110,9 +110,10 @@ __device__ __forceinline__ void cell_coefs(const BlkLev &B, const Coef<T> &cf, i
 // 25.5 ms, 256^3 81.5 -> 80.7 ms.
 constexpr unsigned kPdlCtas = 592;
 __device__ __forceinline__ bool pdl_one_wave() { return gridDim.x * gridDim.y <= kPdlCtas; }
-__device__ __forceinline__ void pdl_wait() {
+// ctas: what one wave holds of the kernel (2*kPdlCtas: 8 light CTAs an SM)
+__device__ __forceinline__ void pdl_wait(unsigned ctas = kPdlCtas) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (pdl_one_wave()) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (gridDim.x * gridDim.y <= ctas) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // A CTA's work: block position and the origin of its tile.  2-D tiles:

@@ -409,18 +409,17 @@ __device__ __forceinline__ bool bc_item(const BlkFld &F, int &ax, int &q, int &s
 // after a diverged solve.
 __global__ void k_bc_walk(const BlkFld *__restrict__ fl, const Tile *__restrict__ tiles,
                           const DomState *__restrict__ ds, int ax, int ly, int mode, int only) {
-  pdl_wait();
   const Tile t = tiles[blockIdx.x];
   const BlkFld &F = fl[t.blk];
-  if (ds[F.dom].rmax > 100.0) return;
   const int comp = only >= 0 ? only : blockIdx.y;
   const bool all = ax < 0;
   int q = t.i0 + threadIdx.x, side, sl, tl;
-  if (!bc_item(F, ax, q, side, sl, tl)) return;
-  const int f = 2 * ax + side;
-  const int pf = F.pface[f];
-  if (!pf) return;
+  const bool item = bc_item(F, ax, q, side, sl, tl);
+  const int f = item ? 2 * ax + side : 0;
+  const int pf = item ? F.pface[f] : 0;
   double *fi = comp_field(F, comp);
+  pdl_wait(2 * kPdlCtas);  // the field table is the call's: no kernel writes it
+  if (!pf || ds[F.dom].rmax > 100.0) return;
   const int s0 = 1, e0 = comp_end(F, comp, ax);
   const long long g = fidx_ax(F, ax, side ? e0 + 1 + ly : s0 - 1 - ly, sl, tl);
   if (mode == 2) {
@@ -548,18 +547,18 @@ __global__ void k_wall_law(const BlkFld *__restrict__ fl, const Tile *__restrict
 __global__ void k_bound_faces(const BlkFld *__restrict__ fl, const Tile *__restrict__ tiles,
                               const DomState *__restrict__ ds, int ax, int ly, double ubulk, int alfabc,
                               int only, double dt, double alfapr) {
-  pdl_wait();
   const Tile t = tiles[blockIdx.x];
   const BlkFld &F = fl[t.blk];
-  if (ds[F.dom].rmax > 100.0) return;
   const int pl = F.pl;
   const int m1 = (ax == 0 ? F.ny : F.nx) + 2 * pl;
   const int comp = only >= 0 ? only : blockIdx.y;  // boundu, boundv or boundw alone, or all three
   int q = t.i0 + threadIdx.x, side, sl, tl;
-  if (!bc_item(F, ax, q, side, sl, tl)) return;
-  const int f = 2 * ax + side;
-  if (!F.wall[f]) return;
+  const bool item = bc_item(F, ax, q, side, sl, tl);
+  const int f = item ? 2 * ax + side : 0;
+  const bool wall = item && F.wall[f];
   const int code = F.bcode[f];
+  pdl_wait(2 * kPdlCtas);
+  if (!wall || ds[F.dom].rmax > 100.0) return;
   const bool normal = comp == ax;
   // 1 constant cv, 2 -mirror, 3 +mirror, 4 copy of the last face,
   // 5 convective outflow, 6 the inlet plane, 7 wall-function update of the
