@@ -1290,8 +1290,10 @@ __global__ void __launch_bounds__(RW_TX *RW_RJ) k_calmas4(const BlkFld *__restri
 // the march, like the component itself.  The next plane's operands load
 // while a plane is computed.  What bounds it: DRAM, 48 B a cell (the three
 // velocities, the start-of-step value, the viscosity, the predicted value).
-// 256^3 in 8 blocks: 193 us a component (4.2 TB/s), against 267 us with six
-// IEEE divisions a cell, every operand loaded anew and none ahead.
+// 256^3 in 8 blocks: 267 us a component with six IEEE divisions a cell, every
+// operand loaded anew and none ahead; 193 us as it stands for 3 CTAs an SM,
+// 175 for 4 (a stage 690 and 635 us; 5: 874, the loads ahead spill; 4 without
+// them: 751).
 template <int COMP>
 struct Rk2Plane {  // what a plane adds to the march at (i, j): C at the plane above, this plane's neighbours
   double ct, cw, ce, cs, cn;  // C(k+1), C(i-1), C(i+1), C(j-1), C(j+1)
@@ -1338,7 +1340,7 @@ __device__ __forceinline__ double rk2_cell(const Rk2Plane<COMP> &v, double cc, d
   return st;
 }
 template <int COMP, int MODE>
-__global__ void __launch_bounds__(RW_TX *RW_RJ, 3) k_rk2nd(const BlkFld *__restrict__ fl,
+__global__ void __launch_bounds__(RW_TX *RW_RJ, MODE == 2 ? 4 : 3) k_rk2nd(const BlkFld *__restrict__ fl,
                                                            const Tile *__restrict__ tiles, double dt, double alfapr,
                                                            int pforce, double forcn) {
   pdl_wait();
@@ -1423,8 +1425,9 @@ __global__ void __launch_bounds__(RW_TX *RW_RJ, 3) k_rk2nd(const BlkFld *__restr
 // The stencils reach three cells each way (pl >= 3).
 // What bounds it: loads through L1 (54 operands a cell) and issue.  COMP
 // fixes the strides' roles at compile time (no indexing of local arrays) and
-// the six quotients take quo: 4 blocks of 90x117x75, 97-113 us a component
-// against 132 us.
+// the six quotients take quo: 4 blocks of 90x117x75, 132 us a component
+// before, 97-113 for 2 CTAs an SM; a stage 413 us, 387 for 4 CTAs and two
+// planes at a time (5: 584, 6: 730, spilled).
 template <int COMP, int MODE>
 __device__ __forceinline__ double rk4_cell(const double *const *vel, const double *OO, const double *VIS,
                                            const long long *st3, const double *h24, const double *r24,
@@ -1463,7 +1466,7 @@ __device__ __forceinline__ double rk4_cell(const double *const *vel, const doubl
   return st;
 }
 template <int COMP, int MODE>
-__global__ void __launch_bounds__(RW_TX *RW_RJ, 2) k_rk4th(const BlkFld *__restrict__ fl,
+__global__ void __launch_bounds__(RW_TX *RW_RJ, 4) k_rk4th(const BlkFld *__restrict__ fl,
                                                            const Tile *__restrict__ tiles, double dt, double alfapr,
                                                            int pforce, double forcn) {
   pdl_wait();
@@ -1486,6 +1489,7 @@ __global__ void __launch_bounds__(RW_TX *RW_RJ, 2) k_rk4th(const BlkFld *__restr
     r24[a] = MODE ? 1.0 / h24[a] : 0.0;
     r12[a] = MODE ? 1.0 / h12[a] : 0.0;
   }
+#pragma unroll 2
   for (int k = t.k0; k <= k1; ++k) {
     const long long c = fidx(F, i, j, k);
     bool bad = false;
@@ -1532,7 +1536,8 @@ __device__ __forceinline__ double weno5(double v1, double v2, double v3, double 
 // terms as k_rk2nd forms them.  Issue bound: both upwind sides take one
 // evaluation on selected differences (a warp holds both signs), and the
 // quotients by h, h*h and the weights' sum need no division each (quo).
-// 128^3 in 8 blocks: 137 us a component against 268 us.
+// 128^3 in 8 blocks: 268 us a component before, 137 for 2 CTAs an SM; a stage
+// 531 us, 447 for 4 (3: 494, 5: 456, 6: 501).
 template <int COMP, int MODE>
 __device__ __forceinline__ double rkw_cell(const double *U, const double *V, const double *W, const double *OO,
                                            const double *VIS, const long long *st3, const int *fx, const int *lim,
@@ -1596,7 +1601,7 @@ __device__ __forceinline__ double rkw_cell(const double *U, const double *V, con
   return st;
 }
 template <int COMP, int MODE>
-__global__ void __launch_bounds__(RW_TX *RW_RJ, 2) k_rkweno(const BlkFld *__restrict__ fl,
+__global__ void __launch_bounds__(RW_TX *RW_RJ, MODE == 2 ? 4 : 3) k_rkweno(const BlkFld *__restrict__ fl,
                                                             const Tile *__restrict__ tiles, int pl_ex, double dt,
                                                             double alfapr, int pforce, double forcn) {
   pdl_wait();
