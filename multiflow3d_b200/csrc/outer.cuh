@@ -1292,8 +1292,8 @@ __global__ void __launch_bounds__(RW_TX *RW_RJ) k_calmas4(const BlkFld *__restri
 // velocities, the start-of-step value, the viscosity, the predicted value).
 // 256^3 in 8 blocks: 267 us a component with six IEEE divisions a cell, every
 // operand loaded anew and none ahead; 193 us as it stands for 3 CTAs an SM,
-// 175 for 4 (a stage 690 and 635 us; 5: 874, the loads ahead spill; 4 without
-// them: 751).
+// 168 for 4 (4.8 TB/s; a stage 690 and 635 us; 5: 874, the loads ahead spill; 4
+// without them: 751).
 template <int COMP>
 struct Rk2Plane {  // what a plane adds to the march at (i, j): C at the plane above, this plane's neighbours
   double ct, cw, ce, cs, cn;  // C(k+1), C(i-1), C(i+1), C(j-1), C(j+1)
