@@ -840,7 +840,10 @@ __global__ void __launch_bounds__(TW_THREADS) k_tdma_wave(const BlkLev *__restri
           const T *ar = rp + b * sl + lane * ld, *av = aa + b * sl + lane * ld;
           T *out = ph + b * sl + lane * ld;
           // batches of TW_CH cells, the next one's operands loaded beside the
-          // chain (reads past the line stay inside the arrays)
+          // chain.  The last batch's load ahead reads past the line: with n >=
+          // TW_CH cells its at most n + TW_CH'th element of `lo` lies within
+          // the 2*(n+2) that begin with lo = ab, the array's last.  Shorter
+          // lines (a level of one or two planes) load nothing ahead.
           T r[TW_CH], z[TW_CH], y[TW_CH];
           auto get = [&](int m0) {
 #pragma unroll
@@ -852,7 +855,7 @@ __global__ void __launch_bounds__(TW_THREADS) k_tdma_wave(const BlkLev *__restri
             }
           };
           const int nf = n / TW_CH * TW_CH;
-          get(0);
+          if (nf > 0) get(0);
           T c = g0[b * lmax + lane];
           for (int m0 = 0; m0 < nf; m0 += TW_CH) {
             T rr[TW_CH], zz[TW_CH], yy[TW_CH];

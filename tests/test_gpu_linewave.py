@@ -56,3 +56,26 @@ def test_line_relaxation_fp32_converges(lib, cuda):
         p = pr.gather([{k: t.cpu().numpy() for k, t in f.items()} for f in d], "p")
         out.append(p - p.mean())
     assert np.linalg.norm(out[1] - out[0]) / np.linalg.norm(out[0]) < 1e-6
+
+
+# levels of one and two planes, where a line is shorter than a batch of the
+# recurrences and its coefficients are the last of the shared memory
+THIN = {
+    "one plane": (9, 6, 1, (1, 1, 1), 1),
+    "two planes, clusters": (40, 33, 2, (1, 1, 1), 1),
+    "a line of seven": (16, 12, 7, (1, 1, 1), 1),
+    "coarsest 4x4x1": (64, 64, 16, (1, 1, 1), 5),
+    "coarsest 4x4x2": (32, 32, 16, (1, 1, 1), 4),
+    "coarsest 8x8x2, two blocks": (32, 32, 8, (2, 1, 1), 3),
+    "coarsest 1x2x4": (16, 32, 64, (1, 1, 1), 5),
+}
+
+
+@pytest.mark.parametrize("shape", sorted(THIN))
+def test_thin_levels_match_oracle(lib, oracle, cuda, shape):
+    nx, ny, nz, (px, py, pz), levels = THIN[shape]
+    pr = Problem(px, py, pz, nx, ny, nz, bc=(P, P, W, W, W, W), ngrid=levels, pl=1, dx=0.017, dy=0.017, dz=0.017)
+    prm = pr.params(mg_itrsch=2, maxcy=3, eps=1e-12)
+    o, g = run_both(lib, oracle, cuda, pr.descriptors(lib), pr.descriptors(oracle), pr.nblocks, prm,
+                    pr.block_fields(seed=53, fourier_modes=0))
+    assert_same(o, g, pr.pl)
