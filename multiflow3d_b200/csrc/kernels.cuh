@@ -150,7 +150,9 @@ enum : int { ERR_TMA_WAIT = 1, ERR_WALL_LAW = 2, ERR_MID_BARRIER = 3, ERR_SIP_WA
 // declares that many more bytes on its first plane's barrier than its
 // copies deliver.  That barrier's phase then never completes: the bounded
 // wait gives up after kMaxWaitNs, records ERR_TMA_WAIT and the CTA leaves,
-// its copies long since landed.  Zero (no effect) unless a test sets it.
+// its copies long since landed.  A k_sip_subst launch that sees it takes it
+// too: its first warp withholds its values, and the warps that wait for them
+// give up.  Zero (no effect) unless a test sets it.
 __device__ int g_test_extra_tx = 0;
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }

@@ -260,20 +260,25 @@ struct SipShared {
 };
 static inline size_t sip_smem(int warps, int R) { return sizeof(SipShared) + (size_t)warps * R * 33 * sizeof(double); }
 
-// a waiting warp's look at the clock: false (and *err set) after kMaxWaitNs
+// A waiting warp's look at the clock, lane 0's for all: the lanes of a warp
+// vote and shuffle together, so they must give up together.  False (and *err
+// set) after kMaxWaitNs.
 __device__ __noinline__ bool sip_patience(unsigned long long &t0, int *err) {
-  const unsigned long long t = global_ns();
+  const unsigned long long t = __shfl_sync(0xffffffffu, global_ns(), 0);
   if (t0 == 0) t0 = t;
   if (t - t0 <= kMaxWaitNs) return true;
   atomicExch(err, ERR_SIP_WAIT);
   return false;
 }
-// until *p >= need (seen: the last value read), the same for all lanes
+// until every lane has read *p >= need (seen: the least of the last values
+// read), the same for all lanes
 __device__ __forceinline__ bool sip_credit(const int *p, int need, int &seen, bool cluster, int *err) {
   unsigned long long t0 = 0;
   while (seen < need) {
-    if (cluster) asm volatile("ld.acquire.cluster.shared::cta.s32 %0, [%1];" : "=r"(seen) : "r"(smem_u32(p)) : "memory");
-    else asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(seen) : "r"(smem_u32(p)) : "memory");
+    int v;
+    if (cluster) asm volatile("ld.acquire.cluster.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
+    else asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
+    seen = __reduce_min_sync(0xffffffffu, v);
     if (seen < need && !sip_patience(t0, err)) return false;
   }
   return true;
@@ -426,6 +431,9 @@ __device__ __forceinline__ bool sip_pass(const SipBlk &S, SipShared &sh, int war
 template <int W, int D, bool RING>
 __global__ void __launch_bounds__(32 * W) k_sip_subst(const SipBlk *__restrict__ sb,
                                                       const SipCtl *__restrict__ ctl, int cl, int *err) {
+  // testing aid: the first warp of the first block may be told to withhold its values
+  const bool first = blockIdx.x == 0 && threadIdx.x < 32;
+  const int hold = first && threadIdx.x == 0 ? *(volatile int *)&g_test_extra_tx : 0;
   pdl_wait();
   if (!ctl->run) return;
   extern __shared__ __align__(16) unsigned char sip_dyn[];
@@ -454,7 +462,8 @@ __global__ void __launch_bounds__(32 * W) k_sip_subst(const SipBlk *__restrict__
   };
   clear();
   bool ok = true;
-  if (mine) {
+  if (first) ok = __shfl_sync(0xffffffffu, hold ? atomicExch(&g_test_extra_tx, 0) : 0, 0) == 0;
+  if (mine && ok) {
     const bool up = jr < nr - 1;  // the row above is this CTA's
     ok = sip_pass<true, W, D, RING>(S, sh, warp, nw, q, lane, j,
                                     above ? above->across(q, R) : up ? sh.across(warp + nseg, R) : nullptr,

@@ -5,8 +5,11 @@ longer and shorter than the rings, 16 and 32 warps a CTA, and planes past
 that (a launch per hyperplane)."""
 import pytest
 
+from multiflow3d_b200 import abi
 from multiflow3d_b200.problems import Problem, WALL
+from multiflow3d_b200.solver import Projection
 from test_gpu_edges import run_both, assert_same
+from test_gpu_failures import _dev, _solve
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +39,31 @@ def test_substitution_launches_match_oracle(lib, oracle, cuda, plane):
                     pr.block_fields(seed=44, fourier_modes=0))
     assert o[0] in (0, 1)
     assert_same(o, g, pr.pl)
+
+
+@pytest.mark.parametrize("plane", ["full segments", "32 warps", "lines past the shared memory",
+                                   "two segments, the second one lane", "two blocks, short last slab"])
+def test_withheld_value_times_out(lib, cuda, plane):
+    """The first row segment withholds its values: the warps that wait for them,
+    or for room in a ring, give up within their limit (2 s), each as a whole, the
+    call returns MF3D_E_TIMEOUT, and the next call on the context equals a fresh
+    context's."""
+    nx, ny, nz, (px, py, pz), nswp = PLANES[plane]
+    pr = Problem(px, py, pz, nx, ny, nz, bc=(WALL,) * 6, ngrid=1, pl=1, dx=0.013, dy=0.013, dz=0.013)
+    prm = pr.params(maxcy=3, eps=1e-9, solver=1, nswp=nswp)
+    host = pr.block_fields(seed=45, fourier_modes=0)
+    proj = Projection(pr.descriptors(lib), prm, lib)
+    assert lib.mf3d_test_stall_copy(0, 16) == abi.MF3D_OK
+    st, _, _ = _solve(lib, proj, _dev(pr, host, cuda), prm.maxcy)
+    lib.mf3d_test_stall_copy(0, 0)
+    assert st == abi.MF3D_E_TIMEOUT, st
+    assert "time limit" in abi.last_error(lib)
+    out = []
+    for call in (proj, Projection(pr.descriptors(lib), prm, lib)):
+        d = _dev(pr, host, cuda)
+        st, info, hist = _solve(lib, call, d, prm.maxcy)
+        call.close()
+        out.append((st, info.iter, hist.tolist(), [f["p"].cpu() for f in d]))
+    assert out[0][:3] == out[1][:3]
+    for a, b in zip(out[0][3], out[1][3]):
+        assert a.equal(b)
