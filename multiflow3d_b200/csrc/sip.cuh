@@ -260,15 +260,20 @@ struct SipShared {
 };
 static inline size_t sip_smem(int warps, int R) { return sizeof(SipShared) + (size_t)warps * R * 33 * sizeof(double); }
 
-// A waiting warp's look at the clock, lane 0's for all: the lanes of a warp
-// vote and shuffle together, so they must give up together.  False (and *err
-// set) after kMaxWaitNs.
-__device__ __noinline__ bool sip_patience(unsigned long long &t0, int *err) {
-  const unsigned long long t = __shfl_sync(0xffffffffu, global_ns(), 0);
-  if (t0 == 0) t0 = t;
-  if (t - t0 <= kMaxWaitNs) return true;
+// A waiting lane's look at the clock.  t0: when it began to wait (0: now),
+// which it returns; 0 (and *err set) after kMaxWaitNs.
+__device__ __noinline__ unsigned long long sip_patience(unsigned long long t0, int *err) {
+  const unsigned long long t = global_ns();
+  if (t0 == 0) return t;
+  if (t - t0 <= kMaxWaitNs) return t0;
   atomicExch(err, ERR_SIP_WAIT);
-  return false;
+  return 0;
+}
+// Whether the warp waits on.  Its lanes vote and shuffle together, so all of
+// them give up when one does, whatever times they read.
+__device__ __forceinline__ bool sip_wait_on(unsigned long long &t0, int *err) {
+  t0 = sip_patience(t0, err);
+  return __all_sync(0xffffffffu, t0 != 0);
 }
 // until every lane has read *p >= need (seen: the least of the last values
 // read), the same for all lanes
@@ -279,7 +284,7 @@ __device__ __forceinline__ bool sip_credit(const int *p, int need, int &seen, bo
     if (cluster) asm volatile("ld.acquire.cluster.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
     else asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
     seen = __reduce_min_sync(0xffffffffu, v);
-    if (seen < need && !sip_patience(t0, err)) return false;
+    if (seen < need && !sip_wait_on(t0, err)) return false;
   }
   return true;
 }
@@ -336,7 +341,7 @@ __device__ __forceinline__ bool sip_pass(const SipBlk &S, SipShared &sh, int war
             nb[d] = __longlong_as_double(v);
           }
           if (__all_sync(0xffffffffu, there)) break;
-          if (!sip_patience(t0, err)) return false;
+          if (!sip_wait_on(t0, err)) return false;
         }
         t0 = 0;
         if (RING)
@@ -357,7 +362,7 @@ __device__ __forceinline__ bool sip_pass(const SipBlk &S, SipShared &sh, int war
               }
             }
           if (__all_sync(0xffffffffu, there)) break;
-          if (!sip_patience(t0, err)) return false;
+          if (!sip_wait_on(t0, err)) return false;
         }
         t0 = 0;
         if (RING && takes)
