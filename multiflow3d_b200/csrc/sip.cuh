@@ -44,8 +44,11 @@ struct SipBlk {
 // steps of a row segment: nz + 31, in whole pairs of chunks (k_sip_subst)
 constexpr int SIP_K = 4;  // steps per chunk
 __host__ __device__ inline int sip_steps(int nz) { return (nz + 31 + 2 * SIP_K - 1) / (2 * SIP_K) * (2 * SIP_K); }
+__device__ __forceinline__ long long sip_plain(const SipBlk &S, int i, int j, int k) {
+  return ((long long)k * (S.ny + 2) + j) * (S.nx + 2) + i;
+}
 __device__ __forceinline__ long long sip_idx(const SipBlk &S, int i, int j, int k) {
-  if (!S.nseg) return ((long long)k * (S.ny + 2) + j) * (S.nx + 2) + i;
+  if (!S.nseg) return sip_plain(S, i, j, k);
   const int l = (i - 1) & 31;
   return (((long long)(j - 1) * S.nseg + ((i - 1) >> 5)) * sip_steps(S.nz) + (k - 1 + l)) * 32 + l;
 }
@@ -176,21 +179,25 @@ __global__ void k_sip_sum(const double *__restrict__ part, int n, SipCtl *__rest
   ctl->next = (rsm <= 0.001 || reldif <= 0.00001) ? 0 : 1;
 }
 
-// Forward substitution on hyperplane h (sipsol.for:149-157).
+// Forward substitution on hyperplane h (sipsol.for:149-157).  `run` is loaded
+// beside the operands and looked at before the store: a launch is a chain of
+// loads, and one more ahead of them cost 0.6 us of 2.3 (96x96x64: 27.8 ms for
+// 6 calls of 4 sweeps, 35.1 with it).
 __global__ void k_sip_forward(const SipBlk *__restrict__ sb, const Tile *__restrict__ tiles, int h,
                               const SipCtl *__restrict__ ctl) {
   pdl_wait();
-  if (!ctl->run) return;
+  const int run = ctl->run;
   const Tile t = tiles[blockIdx.x];
   const SipBlk S = sb[t.blk];
   const int q = t.i0 + threadIdx.x;
   if (q >= S.nx * S.ny) return;
   const int i = q % S.nx + 1, j = q / S.nx + 1, k = h - i - j;
   if (k < 1 || k > S.nz) return;
-  const long long c = sip_idx(S, i, j, k);
-  S.res[c] = (S.res[c] - S.lb[c] * S.res[sip_idx(S, i, j, k - 1)] - S.lw[c] * S.res[sip_idx(S, i - 1, j, k)] -
-              S.ls[c] * S.res[sip_idx(S, i, j - 1, k)]) *
-             S.lpr[c];
+  const long long c = sip_plain(S, i, j, k);
+  const double r = (S.res[c] - S.lb[c] * S.res[sip_plain(S, i, j, k - 1)] - S.lw[c] * S.res[sip_plain(S, i - 1, j, k)] -
+                    S.ls[c] * S.res[sip_plain(S, i, j - 1, k)]) *
+                   S.lpr[c];
+  if (run) S.res[c] = r;
 }
 
 // Backward substitution on hyperplane h and the correction of pp
@@ -198,20 +205,23 @@ __global__ void k_sip_forward(const SipBlk *__restrict__ sb, const Tile *__restr
 __global__ void k_sip_backward(const SipBlk *__restrict__ sb, const BlkLev *__restrict__ bl,
                                const Tile *__restrict__ tiles, int h, const SipCtl *__restrict__ ctl) {
   pdl_wait();
-  if (!ctl->run) return;
+  const int run = ctl->run;
   const Tile t = tiles[blockIdx.x];
   const SipBlk S = sb[t.blk];
   const int q = t.i0 + threadIdx.x;
   if (q >= S.nx * S.ny) return;
   const int i = q % S.nx + 1, j = q / S.nx + 1, k = h - i - j;
   if (k < 1 || k > S.nz) return;
-  const long long c = sip_idx(S, i, j, k);
-  const double r = S.res[c] - S.un[c] * S.res[sip_idx(S, i, j + 1, k)] - S.ue[c] * S.res[sip_idx(S, i + 1, j, k)] -
-                   S.ut[c] * S.res[sip_idx(S, i, j, k + 1)];
-  S.res[c] = r;
+  const long long c = sip_plain(S, i, j, k);
+  const double r = S.res[c] - S.un[c] * S.res[sip_plain(S, i, j + 1, k)] - S.ue[c] * S.res[sip_plain(S, i + 1, j, k)] -
+                   S.ut[c] * S.res[sip_plain(S, i, j, k + 1)];
   double *fi = phi_of<double>(bl[t.blk]);
   const long long e = cell_off(bl[t.blk], i, j, k);
-  fi[e] = fi[e] + r;
+  const double f = fi[e] + r;
+  if (run) {
+    S.res[c] = r;
+    fi[e] = f;
+  }
 }
 
 // Both substitutions of every block in one launch.  A block is a cluster of
