@@ -7,12 +7,14 @@
 // hyperplane i+j+k = h can be formed at once with exactly the reference's
 // operands and operation order.  Where a block's rows fit one cluster's
 // warps, both substitutions run in one launch in which every warp carries a
-// row segment and waits for its neighbours alone (k_sip_subst); larger planes
-// take a launch per hyperplane, the whole sweep captured once in a CUDA
-// graph.  The factors and the residual live in per-block arrays, for the
-// hyperplane launches over the ghost-inclusive box, i fastest, zero outside
-// the interior (the reference zeroes its arrays and only ever writes interior
-// cells), for k_sip_subst in the order in which its warps read them (SipBlk).
+// row segment and waits for its neighbours alone (k_sip_subst).  Small planes
+// that this suits less - narrow and tall ones, very many blocks - are walked
+// by one CTA each, hyperplane by hyperplane (k_sip_subst_col, _block), and
+// larger planes take a launch per hyperplane, the whole sweep captured once
+// in a CUDA graph.  The factors and the residual live in per-block arrays,
+// for k_sip_subst in the order in which its warps read them (SipBlk), else
+// over the ghost-inclusive box, i fastest, zero outside the interior (the
+// reference zeroes its arrays and only ever writes interior cells).
 // The correction pp is the level-1 phi of the
 // multigrid storage, so the pressure update, the halo refresh of pp
 // (exchange(44): its face values are the multigrid halo's) and
@@ -519,6 +521,131 @@ __global__ void __launch_bounds__(RW_TX *RW_RJ) k_sip_add(const SipBlk *__restri
   }
 }
 
+// Both substitutions of a block in one CTA: its hyperplanes one after
+// another, a CTA barrier between them (a block's recurrences never reach
+// into another block).  For small blocks, where a hyperplane holds a few
+// thousand cells at most, this replaces 2*(nx+ny+nz-2) launches per sweep
+// by one; the per-cell arithmetic is k_sip_forward's and k_sip_backward's.
+__global__ void __launch_bounds__(1024) k_sip_subst_block(const SipBlk *__restrict__ sb,
+                                                          const BlkLev *__restrict__ bl,
+                                                          const SipCtl *__restrict__ ctl) {
+  pdl_wait();
+  if (!ctl->run) return;
+  const SipBlk S = sb[blockIdx.x];
+  const BlkLev &B = bl[blockIdx.x];
+  double *fi = phi_of<double>(B);
+  const int hmax = S.nx + S.ny + S.nz, pairs = S.nx * S.ny;
+  for (int h = 3; h <= hmax; ++h) {
+    for (int q = threadIdx.x; q < pairs; q += blockDim.x) {
+      const int i = q % S.nx + 1, j = q / S.nx + 1, k = h - i - j;
+      if (k < 1 || k > S.nz) continue;
+      const long long c = sip_plain(S, i, j, k);
+      S.res[c] = (S.res[c] - S.lb[c] * S.res[sip_plain(S, i, j, k - 1)] - S.lw[c] * S.res[sip_plain(S, i - 1, j, k)] -
+                  S.ls[c] * S.res[sip_plain(S, i, j - 1, k)]) *
+                 S.lpr[c];
+    }
+    __syncthreads();
+  }
+  for (int h = hmax; h >= 3; --h) {
+    for (int q = threadIdx.x; q < pairs; q += blockDim.x) {
+      const int i = q % S.nx + 1, j = q / S.nx + 1, k = h - i - j;
+      if (k < 1 || k > S.nz) continue;
+      const long long c = sip_plain(S, i, j, k);
+      const double r = S.res[c] - S.un[c] * S.res[sip_plain(S, i, j + 1, k)] -
+                       S.ue[c] * S.res[sip_plain(S, i + 1, j, k)] - S.ut[c] * S.res[sip_plain(S, i, j, k + 1)];
+      S.res[c] = r;
+      const long long e = cell_off(B, i, j, k);
+      fi[e] = fi[e] + r;
+    }
+    __syncthreads();
+  }
+}
+
+// The same two substitutions with one thread per (i, j) column, for blocks
+// of at most 1024 columns.  At hyperplane h column (i, j) holds cell
+// k = h-i-j: the cell below is its own previous value (a register), and
+// the cells west and south (forward) or east and north (backward) at the
+// same k were formed by those columns one hyperplane earlier and wait in a
+// shared-memory plane.  Each hyperplane is then two CTA barriers and no
+// dependent global load; the operands of the next cell are loaded one step
+// ahead.  The arithmetic is the reference's, operand for operand.
+__global__ void __launch_bounds__(1024) k_sip_subst_col(const SipBlk *__restrict__ sb,
+                                                        const BlkLev *__restrict__ bl,
+                                                        const SipCtl *__restrict__ ctl) {
+  pdl_wait();
+  if (!ctl->run) return;
+  extern __shared__ double plane[];  // (ny+2) x (nx+2), zero border
+  const SipBlk S = sb[blockIdx.x];
+  const BlkLev &B = bl[blockIdx.x];
+  double *fi = phi_of<double>(B);
+  const int nx = S.nx, ny = S.ny, nz = S.nz, px = nx + 2;
+  const int tid = threadIdx.x;
+  for (int q = tid; q < (ny + 2) * px; q += blockDim.x) plane[q] = 0.0;
+  const bool col = tid < nx * ny;
+  const int i = tid % nx + 1, j = tid / nx + 1;
+  const int hmax = nx + ny + nz;
+  __syncthreads();
+  // forward: res = (res - lb*res(k-1) - lw*res(i-1) - ls*res(j-1)) * lpr
+  double below = 0.0;
+  int kn = 3 - i - j;  // k at the next step
+  double nres = 0.0, nlb = 0.0, nlw = 0.0, nls = 0.0, nlpr = 0.0;
+  auto fetch_f = [&](int k) {
+    if (col && k >= 1 && k <= nz) {
+      const long long c = sip_plain(S, i, j, k);
+      nres = S.res[c]; nlb = S.lb[c]; nlw = S.lw[c]; nls = S.ls[c]; nlpr = S.lpr[c];
+    }
+  };
+  fetch_f(kn);
+  for (int h = 3; h <= hmax; ++h) {
+    const int k = h - i - j;
+    const bool act = col && k >= 1 && k <= nz;
+    double v = 0.0;
+    if (act) {
+      const double w = plane[j * px + i - 1], so = plane[(j - 1) * px + i];
+      v = (nres - nlb * below - nlw * w - nls * so) * nlpr;
+    }
+    fetch_f(k + 1);
+    __syncthreads();
+    if (act) {
+      plane[j * px + i] = v;
+      S.res[sip_plain(S, i, j, k)] = v;
+      below = v;
+    }
+    __syncthreads();
+  }
+  // backward: res = res - un*res(j+1) - ue*res(i+1) - ut*res(k+1); fi += res
+  for (int q = tid; q < (ny + 2) * px; q += blockDim.x) plane[q] = 0.0;
+  __syncthreads();
+  double above = 0.0;
+  double bres = 0.0, bun = 0.0, bue = 0.0, but = 0.0;
+  auto fetch_b = [&](int k) {
+    if (col && k >= 1 && k <= nz) {
+      const long long c = sip_plain(S, i, j, k);
+      bres = S.res[c]; bun = S.un[c]; bue = S.ue[c]; but = S.ut[c];
+    }
+  };
+  fetch_b(hmax - i - j);
+  for (int h = hmax; h >= 3; --h) {
+    const int k = h - i - j;
+    const bool act = col && k >= 1 && k <= nz;
+    double r = 0.0;
+    if (act) {
+      const double no = plane[(j + 1) * px + i], ea = plane[j * px + i + 1];
+      r = bres - bun * no - bue * ea - but * above;
+    }
+    fetch_b(k - 1);
+    __syncthreads();
+    if (act) {
+      plane[j * px + i] = r;
+      S.res[sip_plain(S, i, j, k)] = r;
+      const long long e = cell_off(B, i, j, k);
+      fi[e] = fi[e] + r;
+      above = r;
+    }
+    __syncthreads();
+  }
+}
+
 constexpr size_t kSipSmem = 220 * 1024;
 constexpr int kSipSlabs = 8;  // CTAs per block of k_sip_subst at most (portable cluster size)
 // CTAs per block of k_sip_subst with at most W warps each: as many as leave
@@ -541,6 +668,56 @@ static int sip_slabs(const std::vector<SipBlk> &hb, int nsm, int W, int &warps) 
   return cl;
 }
 
+constexpr int kSipBlockCells = 4096;  // columns of a plane that one CTA walks at most
+
+// Which way for a view.  k_sip_subst's time is its chain, the rows, row
+// segments and chunks of steps one after the other, times the waves its
+// clusters need; a CTA's is its hyperplanes, at a price that grows with the
+// columns at work, times the waves of blocks; the launches' is theirs, growing
+// with their CTAs.  k_sip_subst falls behind on narrow tall planes (one or two
+// lanes of 32 at work, 17 and more warps a CTA) and on more clusters than the
+// device holds.  The estimates are microseconds a sweep, fitted to all three on
+// shapes that k_sip_subst takes (1..400 x 4..256 columns, 3..200 planes, 1..216
+// blocks; 9 to 12 % rms).  Over 479 random ones of them the choice takes 0.6 %
+// longer than the better way on average and 26 % at worst, always k_sip_subst
+// up to 8.4 times longer, never up to 12 times.  4x130x8 in 200 blocks, 2 calls
+// of 4 sweeps: 37 ms and 8.4; 32x32x32 in 64 blocks: 3.1 and 4.8 ms.
+static double sip_rows_us(const std::vector<SipBlk> &hb, int warps, bool ring, int clusters) {
+  double chain = 0.0, slots = 0.0;
+  int chunks = 0;  // of a row segment: the warps at work at once at most
+  for (const auto &b : hb) {
+    const int nseg = (b.nx + 31) / 32, c = sip_steps(b.nz) / SIP_K;
+    chain = std::max(chain, b.ny + 17.0 * (nseg - 1) + c);
+    chunks = std::max(chunks, c);
+    slots += 32.0 * b.ny * nseg * sip_steps(b.nz);
+  }
+  const int nb = (int)hb.size(), waves = (nb + clusters - 1) / clusters;
+  const double price = warps > 16 ? 0.21 + 0.03 * std::min(warps, chunks) + 0.025 * warps : ring ? 0.73 : 0.38;
+  return 43.0 + waves * 2.0 * chain * price + 1.2 * nb + 3.7e-5 * slots;
+}
+static double sip_cta_us(const std::vector<SipBlk> &hb, int nsm) {
+  double planes = 0.0, price = 0.0, cells = 0.0;
+  for (const auto &b : hb) {
+    const double cols = (double)b.nx * b.ny, h = b.nx + b.ny + b.nz, at_work = cols * b.nz / h;
+    planes = std::max(planes, h - 2.0);
+    price = std::max(price, cols <= 1024 ? 0.58 + 1.9e-3 * at_work
+                                         : 0.74 + 3.1e-3 * at_work + 1.5e-4 * cols + 8.2e-4 * b.nx);
+    cells += cols * b.nz;
+  }
+  const int nb = (int)hb.size(), waves = (nb + nsm - 1) / nsm;
+  return 27.0 + waves * 2.0 * planes * price * (1.0 + 0.48 * std::min(nb, nsm) / nsm) + 1.4 * nb + 7.8e-5 * cells;
+}
+static double sip_launch_us(const std::vector<SipBlk> &hb) {
+  double planes = 0.0, cols = 0.0, at_work = 0.0;
+  for (const auto &b : hb) {
+    const double c = (double)b.nx * b.ny, h = b.nx + b.ny + b.nz;
+    planes = std::max(planes, h - 2.0);
+    cols += c;
+    at_work += c * b.nz / h;
+  }
+  return 20.0 + 2.0 * planes * (1.9 + 1.8e-6 * cols + 9.4e-5 * at_work) + 1.5 * (double)hb.size();
+}
+
 // ---------------------------------------------------------------------------
 // Host side.
 // ---------------------------------------------------------------------------
@@ -551,9 +728,11 @@ struct SipState {
   int n_ij = 0, hmax = 0;
   DevBuf<double> part;
   DevBuf<SipCtl> ctl;
-  int cl = 0, warps = 0;               // k_sip_subst: CTAs per block (0: hyperplane launches), warps per CTA,
+  int cl = 0, warps = 0;               // k_sip_subst: CTAs per block (0: another way), warps per CTA,
   size_t smem = 0;                     // its shared memory and variant
   void (*subst)(const SipBlk *, const SipCtl *, int, int *) = nullptr;
+  void (*cta)(const SipBlk *, const BlkLev *, const SipCtl *) = nullptr;  // one CTA per block, or null
+  size_t cta_smem = 0;
   cudaGraphExec_t sweep = nullptr;     // hyperplane launches: forward + backward substitutions
   ~SipState() {
     if (sweep) cudaGraphExecDestroy(sweep);
@@ -575,9 +754,10 @@ static int sip_prepare(mf3d_ctx *C, View &V) {
     items.push_back((long long)d.nx * d.ny);
     S->hmax = std::max(S->hmax, d.nx + d.ny + d.nz);
   }
-  // one launch for the substitutions where the rows fit a cluster and the
-  // arrays in its order (sip_steps of 32 columns a row segment) leave half
-  // of the free memory
+  // one launch for the substitutions: k_sip_subst where the rows fit a cluster
+  // and the arrays in its order (sip_steps of 32 columns a row segment) leave
+  // half of the free memory, or a CTA per block, whichever is estimated the
+  // fastest, these two or the launches
   auto elems = [](const SipBlk &b, int nseg) {
     return nseg ? (size_t)b.ny * nseg * sip_steps(b.nz) * 32 : (size_t)(b.nx + 2) * (b.ny + 2) * (b.nz + 2);
   };
@@ -588,6 +768,43 @@ static int sip_prepare(mf3d_ctx *C, View &V) {
   size_t need = 0, room = 0, all = 0;
   for (const auto &b : hb) need += 8 * sizeof(double) * elems(b, (b.nx + 31) / 32);
   if (S->cl && (cudaMemGetInfo(&room, &all) != cudaSuccess || need > room / 2)) S->cl = 0;
+  int clusters = 0;  // resident at once
+  bool ring = false;
+  if (S->cl) {
+    int T = 1;
+    for (const auto &b : hb) T = std::max(T, sip_steps(b.nz));
+    ring = S->warps > 16 || sip_smem(S->warps, T) > kSipSmem;
+    S->subst = S->warps <= 8    ? (ring ? k_sip_subst<8, 8, true> : k_sip_subst<8, 8, false>)
+               : S->warps <= 16 ? (ring ? k_sip_subst<16, 8, true> : k_sip_subst<16, 8, false>)
+                                : k_sip_subst<32, 4, true>;
+    S->smem = sip_smem(S->warps, ring ? sip_ring(S->warps <= 8 ? 8 : S->warps <= 16 ? 16 : 32) : T);
+    CK(cudaFuncSetAttribute(S->subst, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSipSmem));
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)S->cl;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nb * S->cl));
+    cfg.blockDim = dim3(32 * S->warps);
+    cfg.dynamicSmemBytes = S->smem;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&clusters, S->subst, &cfg) != cudaSuccess || clusters < 1) {
+      cudaGetLastError();
+      S->cl = 0;
+    }
+  }
+  int cols = 1, px = 1;  // columns of the largest plane; its size with a border
+  for (const auto &b : hb) {
+    cols = std::max(cols, b.nx * b.ny);
+    px = std::max(px, (b.nx + 2) * (b.ny + 2));
+  }
+  const double by_launch = sip_launch_us(hb), by_cta = cols <= kSipBlockCells ? sip_cta_us(hb, C->nsm) : 1e300;
+  if (S->cl && sip_rows_us(hb, S->warps, ring, clusters) > 0.95 * (0.75 * by_cta <= by_launch ? by_cta : by_launch)) S->cl = 0;
+  if (!S->cl && 0.75 * by_cta <= by_launch) {  // the launches only where they are clearly faster
+    S->cta = cols <= 1024 ? k_sip_subst_col : k_sip_subst_block;
+    S->cta_smem = cols <= 1024 ? (size_t)px * sizeof(double) : 0;
+  }
   for (int b = 0; b < nb; ++b) {
     const int nseg = S->cl ? (hb[b].nx + 31) / 32 : 0;
     const size_t n = elems(hb[b], nseg);
@@ -610,16 +827,7 @@ static int sip_prepare(mf3d_ctx *C, View &V) {
   const BlkLev *L1 = V.lv[1].tab.p;
   for (int h = 3; h <= S->hmax; ++h)
     launch(k_sip_factor, S->n_ij, kTile, 0, s, S->sb.p, L1, S->t_ij.p, h);
-  if (S->cl) {
-    int T = 1;
-    for (const auto &b : hb) T = std::max(T, sip_steps(b.nz));
-    const bool ring = sip_smem(S->warps, T) > kSipSmem;
-    S->subst = S->warps <= 8    ? (ring ? k_sip_subst<8, 8, true> : k_sip_subst<8, 8, false>)
-               : S->warps <= 16 ? (ring ? k_sip_subst<16, 8, true> : k_sip_subst<16, 8, false>)
-                                : k_sip_subst<32, 4, true>;
-    S->smem = sip_smem(S->warps, ring || S->warps > 16 ? sip_ring(S->warps <= 8 ? 8 : S->warps <= 16 ? 16 : 32) : T);
-    CK(cudaFuncSetAttribute(S->subst, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSipSmem));
-  } else {
+  if (!S->cl && !S->cta) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int h = 3; h <= S->hmax; ++h)
@@ -660,11 +868,13 @@ static int sip_solve(mf3d_ctx *C, View &V, bool first_call) {
       launch_cl(S.subst, (int)V.blk.size() * S.cl, 32 * S.warps, S.smem, s, S.cl, S.sb.p, (const SipCtl *)ctl, S.cl,
                 V.err.p);
       launch(k_sip_add, V.n_int, dim3(RW_TX, RW_RJ), 0, s, S.sb.p, L1.tab.p, V.t_int.p, (const SipCtl *)ctl);
+    } else if (S.cta) {
+      launch(S.cta, (int)V.blk.size(), 1024, S.cta_smem, s, S.sb.p, L1.tab.p, (const SipCtl *)ctl);
     } else {
       CK(cudaGraphLaunch(S.sweep, s));
     }
     halo<double>(C, V, 1, SUB_A, &ctl->run);
-    C->launches += 2 + (S.cl ? 2 : 2 * (S.hmax - 2));
+    C->launches += 2 + (S.cl ? 2 : S.cta ? 1 : 2 * (S.hmax - 2));
     if (sweep % kSipAhead == 0 && sweep < C->prm.nswp) {
       int next = 0;
       CK(cudaMemcpyAsync(&next, &ctl->next, sizeof next, cudaMemcpyDeviceToHost, s));

@@ -67,3 +67,44 @@ def test_withheld_value_times_out(lib, cuda, plane):
     assert out[0][:3] == out[1][:3]
     for a, b in zip(out[0][3], out[1][3]):
         assert a.equal(b)
+
+
+def _launches(lib, cuda, cells, blocks, nswp):
+    pr = Problem(*blocks, *cells, bc=(WALL,) * 6, ngrid=1, pl=1, dx=0.013, dy=0.013, dz=0.013)
+    prm = pr.params(maxcy=2, eps=1e-30, solver=1, nswp=nswp)
+    proj = Projection(pr.descriptors(lib), prm, lib)
+    proj.newsolv_mg_device(_dev(pr, pr.block_fields(seed=46, fourier_modes=0), cuda))
+    n = proj.launches
+    proj.close()
+    return n
+
+
+# planes that one CTA walks: past 256 segments, and where the rows' warps would
+# mostly wait (nx, ny, nz, blocks, nswp)
+CTA_PLANES = {
+    "a thread per column": (3, 300, 4, (1, 1, 1), 3),
+    "1024 columns": (4, 256, 2, (1, 1, 1), 2),
+    "a column of 1000 rows": (1, 1000, 3, (1, 1, 1), 2),
+    "several columns a thread": (5, 300, 3, (1, 1, 1), 3),
+    "4096 columns": (2, 2048, 2, (1, 1, 1), 2),
+    "a wide row": (1100, 2, 3, (1, 1, 1), 2),
+    "few lanes, tall": (2, 200, 8, (1, 1, 1), 9),
+    "two tall blocks": (3, 140, 5, (1, 2, 1), 2),
+    "many blocks": (4, 130, 2, (4, 2, 2), 2),
+}
+
+
+@pytest.mark.parametrize("plane", sorted(CTA_PLANES))
+def test_cta_planes_match_oracle(lib, oracle, cuda, plane):
+    nx, ny, nz, (px, py, pz), nswp = CTA_PLANES[plane]
+    pr = Problem(px, py, pz, nx, ny, nz, bc=(WALL,) * 6, ngrid=1, pl=1, dx=0.013, dy=0.013, dz=0.013)
+    prm = pr.params(maxcy=4, eps=1e-9, solver=1, nswp=nswp)
+    o, g = run_both(lib, oracle, cuda, pr.descriptors(lib), pr.descriptors(oracle), pr.nblocks, prm,
+                    pr.block_fields(seed=47, fourier_modes=0))
+    assert_same(o, g, pr.pl)
+    # one launch for both substitutions, which adds to pp as well (k_sip_subst
+    # leaves that to a second launch)
+    if pr.nblocks == 1:
+        rows = _launches(lib, cuda, (32, 32, 5), (1, 1, 1), 2) - _launches(lib, cuda, (32, 32, 5), (1, 1, 1), 1)
+        here = _launches(lib, cuda, (nx, ny, nz), (1, 1, 1), 2) - _launches(lib, cuda, (nx, ny, nz), (1, 1, 1), 1)
+        assert here == rows - 2  # two calls
