@@ -733,9 +733,13 @@ struct SipState {
   void (*subst)(const SipBlk *, const SipCtl *, int, int *) = nullptr;
   void (*cta)(const SipBlk *, const BlkLev *, const SipCtl *) = nullptr;  // one CTA per block, or null
   size_t cta_smem = 0;
-  cudaGraphExec_t sweep = nullptr;     // hyperplane launches: forward + backward substitutions
+  cudaGraphExec_t sweep = nullptr;     // hyperplane launches: forward + backward substitutions,
+  int *next = nullptr;                 // the stopping test's answer on the host (pinned),
+  cudaEvent_t tested = nullptr;        // there once this is recorded
   ~SipState() {
     if (sweep) cudaGraphExecDestroy(sweep);
+    if (tested) cudaEventDestroy(tested);
+    if (next) cudaFreeHost(next);
   }
 };
 
@@ -828,6 +832,8 @@ static int sip_prepare(mf3d_ctx *C, View &V) {
   for (int h = 3; h <= S->hmax; ++h)
     launch(k_sip_factor, S->n_ij, kTile, 0, s, S->sb.p, L1, S->t_ij.p, h);
   if (!S->cl && !S->cta) {
+    CK(cudaMallocHost(&S->next, sizeof(int)));
+    CK(cudaEventCreateWithFlags(&S->tested, cudaEventDisableTiming));
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int h = 3; h <= S->hmax; ++h)
@@ -848,6 +854,9 @@ static int sip_prepare(mf3d_ctx *C, View &V) {
 // sipsol(44): pp := 0, then up to nswp sweeps, the stopping test on the
 // device (SipCtl).  The host queues them without waiting, but looks at the
 // test every kSipAhead sweeps so that a long budget is not queued in vain.
+// A sweep of hyperplane launches, hundreds of them, costs nearly as much when
+// it has nothing to do: there the host reads each test's answer while the
+// substitutions it precedes are running, and queues no sweep past the stop.
 constexpr int kSipAhead = 8;
 static int sip_solve(mf3d_ctx *C, View &V, bool first_call) {
   cudaStream_t s = C->stream;
@@ -871,11 +880,16 @@ static int sip_solve(mf3d_ctx *C, View &V, bool first_call) {
     } else if (S.cta) {
       launch(S.cta, (int)V.blk.size(), 1024, S.cta_smem, s, S.sb.p, L1.tab.p, (const SipCtl *)ctl);
     } else {
+      CK(cudaMemcpyAsync(S.next, &ctl->next, sizeof(int), cudaMemcpyDeviceToHost, s));
+      CK(cudaEventRecord(S.tested, s));
       CK(cudaGraphLaunch(S.sweep, s));
     }
     halo<double>(C, V, 1, SUB_A, &ctl->run);
     C->launches += 2 + (S.cl ? 2 : S.cta ? 1 : 2 * (S.hmax - 2));
-    if (sweep % kSipAhead == 0 && sweep < C->prm.nswp) {
+    if (S.sweep) {
+      CK(cudaEventSynchronize(S.tested));
+      if (!*S.next) break;
+    } else if (sweep % kSipAhead == 0 && sweep < C->prm.nswp) {
       int next = 0;
       CK(cudaMemcpyAsync(&next, &ctl->next, sizeof next, cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));

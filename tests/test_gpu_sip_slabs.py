@@ -108,3 +108,25 @@ def test_cta_planes_match_oracle(lib, oracle, cuda, plane):
         rows = _launches(lib, cuda, (32, 32, 5), (1, 1, 1), 2) - _launches(lib, cuda, (32, 32, 5), (1, 1, 1), 1)
         here = _launches(lib, cuda, (nx, ny, nz), (1, 1, 1), 2) - _launches(lib, cuda, (nx, ny, nz), (1, 1, 1), 1)
         assert here == rows - 2  # two calls
+
+
+def test_no_launches_past_the_stop(lib, cuda):
+    """A call whose sweeps stop before their budget queues no hyperplane launches
+    for the rest: the launches tell the sweeps run, the pressure is that of
+    exactly so many, and one sweep less gives another."""
+    pr = Problem(1, 1, 1, 129, 65, 2, bc=(WALL,) * 6, ngrid=1, pl=1, dx=0.013, dy=0.013, dz=0.013)
+    host = pr.block_fields(seed=48, fourier_modes=0)
+
+    def call(nswp):
+        proj = Projection(pr.descriptors(lib), pr.params(maxcy=1, eps=1e-30, solver=1, nswp=nswp), lib)
+        d = _dev(pr, host, cuda)
+        proj.newsolv_mg_device(d)
+        n = proj.launches
+        proj.close()
+        return n, d[0]["p"].cpu()
+
+    one, two, (many, p) = call(1)[0], call(2)[0], call(400)
+    sweeps, rest = divmod(many - one, two - one)
+    assert rest == 0 and 1 < sweeps < 399
+    assert p.equal(call(sweeps + 1)[1])
+    assert not p.equal(call(sweeps)[1])
