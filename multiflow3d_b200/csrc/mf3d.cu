@@ -13,6 +13,7 @@
 // current mix of resident requests.
 #include <algorithm>
 #include <array>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -2824,6 +2825,10 @@ static int check_device_error(View &V) {
   }
   if (e == ERR_MID_BARRIER) {
     set_error("a grid barrier of the middle-level V-cycle launch did not complete within its time limit");
+    return MF3D_E_TIMEOUT;
+  }
+  if (e == ERR_SIP_WAIT) {
+    set_error("a wait between the warps of the SIP substitutions did not complete within its time limit");
     return MF3D_E_TIMEOUT;
   }
   set_error("a device copy did not complete within its time limit (code " + std::to_string(e) + ")");

@@ -154,11 +154,13 @@ __global__ void __launch_bounds__(RW_TX *RW_RJ) k_sip_residual(const SipBlk *__r
 }
 
 // The per-CTA sums added in index order by one CTA (a fixed tree), then
-// the stopping test of sipsol.for on the sum.
-__global__ void k_sip_sum(const double *__restrict__ part, int n, SipCtl *__restrict__ ctl) {
+// the stopping test of sipsol.for on the sum.  After a wait of the
+// substitutions gave up nothing runs any more: the call has failed.
+__global__ void k_sip_sum(const double *__restrict__ part, int n, SipCtl *__restrict__ ctl,
+                          const int *__restrict__ err) {
   pdl_wait();
   __shared__ double s[1024];
-  const int go = ctl->next;
+  const int go = *err == ERR_SIP_WAIT ? 0 : ctl->next;
   double v = 0.0;
   if (go)
     for (int q = threadIdx.x; q < n; q += blockDim.x) v = v + part[q];
@@ -170,7 +172,10 @@ __global__ void k_sip_sum(const double *__restrict__ part, int n, SipCtl *__rest
   }
   if (threadIdx.x != 0) return;
   ctl->run = go;
-  if (!go) return;
+  if (!go) {
+    ctl->next = 0;
+    return;
+  }
   const double resab = s[0];
   if (ctl->sweeps == 0) ctl->res1 = resab;
   const double rsm = resab / (ctl->res1 + kSipSmall);
@@ -872,7 +877,7 @@ static int sip_solve(mf3d_ctx *C, View &V, bool first_call) {
   for (int sweep = 1; sweep <= C->prm.nswp; ++sweep) {
     launch(k_sip_residual, V.n_int, dim3(RW_TX, RW_RJ), 0, s, S.sb.p, L1.tab.p, V.t_int.p, S.part.p,
            (const SipCtl *)ctl);
-    launch(k_sip_sum, 1, 1024, 0, s, (const double *)S.part.p, V.n_int, ctl);
+    launch(k_sip_sum, 1, 1024, 0, s, (const double *)S.part.p, V.n_int, ctl, (const int *)V.err.p);
     if (S.cl) {
       launch_cl(S.subst, (int)V.blk.size() * S.cl, 32 * S.warps, S.smem, s, S.cl, S.sb.p, (const SipCtl *)ctl, S.cl,
                 V.err.p);
@@ -915,6 +920,8 @@ static int solve_view_sip(mf3d_ctx *C, View &V, const double *dt, const double *
   double rmax = D.rmax0;
   int calls = 0, done = D.done == 2 ? 2 : 0;
   std::vector<double> hh;
+  using Clock = std::chrono::steady_clock;
+  Clock::time_point began = Clock::now();
   for (int iter = 1; iter <= maxcy && done == 0; ++iter) {
     if (iter > 1 && rmax < D.eps) { done = 1; break; }
     if ((st = sip_solve(C, V, calls == 0))) return st;
@@ -929,6 +936,16 @@ static int solve_view_sip(mf3d_ctx *C, View &V, const double *dt, const double *
     unsigned long long bits = 0;
     CK(cudaMemcpyAsync(&bits, V.rmax.p, sizeof bits, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    // a wait that gave up took kMaxWaitNs: only after such a round is its code
+    // read, and collect() then reports it
+    const Clock::time_point now = Clock::now();
+    if (now - began > std::chrono::nanoseconds(kMaxWaitNs / 2)) {
+      int e = 0;
+      CK(cudaMemcpyAsync(&e, V.err.p, sizeof e, cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+      if (e == ERR_SIP_WAIT) break;
+    }
+    began = now;
     std::memcpy(&rmax, &bits, sizeof rmax);
     hh.push_back(rmax);
     if (!(rmax <= 1.7976931348623157e308)) done = 2;

@@ -130,3 +130,21 @@ def test_no_launches_past_the_stop(lib, cuda):
     assert rest == 0 and 1 < sweeps < 399
     assert p.equal(call(sweeps + 1)[1])
     assert not p.equal(call(sweeps)[1])
+
+
+def test_a_timeout_ends_the_call(lib, cuda):
+    """After a wait gave up the call ends with its round, says which wait it was,
+    and runs no further sweeps or rounds on what is left."""
+    pr = Problem(1, 1, 1, 32, 32, 5, bc=(WALL,) * 6, ngrid=1, pl=1, dx=0.013, dy=0.013, dz=0.013)
+    prm = pr.params(maxcy=200, eps=1e-30, solver=1, nswp=20)
+    host = pr.block_fields(seed=49, fourier_modes=0)
+    proj = Projection(pr.descriptors(lib), prm, lib)
+    _solve(lib, proj, _dev(pr, host, cuda), prm.maxcy)
+    whole = proj.launches
+    assert lib.mf3d_test_stall_copy(0, 16) == abi.MF3D_OK
+    st, _, _ = _solve(lib, proj, _dev(pr, host, cuda), prm.maxcy)
+    lib.mf3d_test_stall_copy(0, 0)
+    stalled = proj.launches
+    proj.close()
+    assert st == abi.MF3D_E_TIMEOUT and "SIP" in abi.last_error(lib)
+    assert stalled < whole / 100
