@@ -150,7 +150,8 @@ enum : int { ERR_TMA_WAIT = 1, ERR_WALL_LAW = 2, ERR_MID_BARRIER = 3, ERR_SIP_WA
 // declares that many more bytes on its first plane's barrier than its
 // copies deliver.  That barrier's phase then never completes: the bounded
 // wait gives up after kMaxWaitNs, records ERR_TMA_WAIT and the CTA leaves,
-// its copies long since landed.  A k_sip_subst launch that sees it takes it
+// its copies long since landed.  The plain-load sweep, which copies nothing,
+// takes it in its first thread and waits for the bytes alone (test_stall).  A k_sip_subst launch that sees it takes it
 // too: its first warp withholds its values, and the warps that wait for them
 // give up.  Zero (no effect) unless a test sets it.
 __device__ int g_test_extra_tx = 0;
@@ -194,6 +195,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, int *e
       return false;
     }
   }
+}
+// The testing aid in a kernel without copies: one thread waits for bytes that
+// nothing delivers, and gives up.
+__device__ __noinline__ void test_stall(int *err) {
+  __shared__ __align__(8) uint64_t bar;
+  const unsigned extra = (unsigned)atomicExch(&g_test_extra_tx, 0);
+  if (!extra) return;
+  mbar_init(&bar, 1);
+  mbar_fence_init();
+  mbar_expect_tx(&bar, extra);
+  mbar_wait(&bar, 0, err);
 }
 // 3-D tiled TMA load of one box into shared memory, completing on `bar`.
 // x (innermost) must be a multiple of 16 bytes / element size.
@@ -421,8 +433,10 @@ __global__ void __launch_bounds__(RB_TX *RB_TY) k_rbgs(const BlkLev *__restrict_
 template <typename T, bool FROM_ZERO>
 __global__ void __launch_bounds__(kTile) k_rbgs_small(const BlkLev *__restrict__ bl, const int *__restrict__ pre,
                                                       const int *__restrict__ blocks, int nb,
-                                                      const int *__restrict__ act, int colour) {
+                                                      const int *__restrict__ act, int colour,
+                                                      int *__restrict__ err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int stall = t == 0 ? *(volatile int *)&g_test_extra_tx : 0;  // testing aid
   if (t >= pre[nb]) return pdl_wait();
   int lo = 0, hi = nb - 1;  // last list entry whose first item <= t
   while (lo < hi) {
@@ -448,7 +462,9 @@ __global__ void __launch_bounds__(kTile) k_rbgs_small(const BlkLev *__restrict__
   const bool early = !B.cc && pdl_one_wave();  // (per-cell coefficients: a kernel of the solve formed them)
   if (early) cell_coefs(B, cf, min(i, B.nx), j, k, aw, ae, as, an, ab, at);
   pdl_wait();
-  if (!act[B.dom] || i > B.nx) return;
+  if (!act[B.dom]) return;
+  if (stall) test_stall(err);
+  if (i > B.nx) return;
   if (!early) cell_coefs(B, cf, i, j, k, aw, ae, as, an, ab, at);
   T w = (T)0, e = (T)0, so = (T)0, no = (T)0, bo = (T)0, to = (T)0;
   if (!FROM_ZERO) {

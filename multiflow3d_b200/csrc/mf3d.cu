@@ -108,10 +108,6 @@ static bool injected_alloc_failure() {
   return c == 0;
 }
 
-// Testing aid (mf3d_test_stall_copy): set while a stall is armed.  Small
-// levels then sweep with the TMA kernel too, the one that can stall.
-static std::atomic<bool> g_stall_armed{false};
-
 // A device array.  alloc() keeps the current allocation when it is large
 // enough (rebuilt launch tables reuse their buffers).
 template <typename T>
@@ -991,7 +987,6 @@ struct View {
   cudaGraphExec_t x_loop = nullptr, x_once = nullptr;
   cudaGraphConditionalHandle cond = 0;
   long long launches_per_iter = 0;
-  bool graphs_armed = false;          // captured with g_stall_armed set
   void drop_graphs() {
     if (x_loop) cudaGraphExecDestroy(x_loop);
     if (g_loop) cudaGraphDestroy(g_loop);
@@ -1980,18 +1975,20 @@ static void relax(mf3d_ctx *C, View &V, int g, int q, int it, bool from_zero, bo
       const bool skip_red = fz && red_done;  // the restriction formed the red half-sweep
       prof_begin(C, fz ? 0 : pk, 3 * half);
       const dim3 grid(L.n_sweep[q]), cta(RB_TX, RB_TY);
-      if (L.small && (C->prm.lsm || !g_stall_armed)) {
+      if (L.small) {
         const int g2 = grid_of(L.small_items[q], kTile);
         if (skip_red)
           ;
         else if (fz)
-          launch(k_rbgs_small<T, true>, g2, kTile, 0, C->stream, L.tab.p, L.spre[q].p, L.list[q].p, L.n_list[q], V.act.p, 0);
+          launch(k_rbgs_small<T, true>, g2, kTile, 0, C->stream, L.tab.p, L.spre[q].p, L.list[q].p, L.n_list[q], V.act.p,
+                 0, V.err.p);
         else
           launch(k_rbgs_small<T, false>, g2, kTile, 0, C->stream, L.tab.p, L.spre[q].p, L.list[q].p, L.n_list[q], V.act.p,
-                                                             0);
+                 0, V.err.p);
         prof_end(C, fz ? 0 : pk);
         prof_begin(C, pk, 3 * half);
-        launch(k_rbgs_small<T, false>, g2, kTile, 0, C->stream, L.tab.p, L.spre[q].p, L.list[q].p, L.n_list[q], V.act.p, 1);
+        launch(k_rbgs_small<T, false>, g2, kTile, 0, C->stream, L.tab.p, L.spre[q].p, L.list[q].p, L.n_list[q], V.act.p, 1,
+               V.err.p);
         prof_end(C, pk);
         C->launches += skip_red ? 1 : 2;
         halo<T>(C, V, g, q);
@@ -2876,10 +2873,6 @@ static int solve_view(mf3d_ctx *C, View &V, const double *dt, const double *alfa
   long long iters_run = 0;
   if (maxcy > 0) {
     if (C->use_graph && C->prof_kind == 0) {
-      if (V.graphs_armed != g_stall_armed) {
-        V.drop_graphs();
-        V.graphs_armed = g_stall_armed;
-      }
       if ((st = build_graphs<T>(C, V)) && V.mid_on) {
         // a driver that does not capture the cooperative middle-level launch
         // into the loop graph: the launch path instead
@@ -4031,7 +4024,6 @@ int mf3d_test_stall_copy(int device, int bytes) {
   if (cudaSetDevice(device) != cudaSuccess) { mf3d::set_error("cudaSetDevice failed"); return MF3D_E_CUDA; }
   const cudaError_t e = cudaMemcpyToSymbol(mf3d::g_test_extra_tx, &bytes, sizeof(int));
   if (e != cudaSuccess) { mf3d::set_error(std::string("mf3d_test_stall_copy: ") + cudaGetErrorString(e)); return MF3D_E_CUDA; }
-  mf3d::g_stall_armed = bytes > 0;
   return MF3D_OK;
 }
 

@@ -149,3 +149,35 @@ def test_stalled_copy_times_out(lib, oracle, cuda):
     assert st2 == st_ref and info2.iter == info_ref.iter
     assert np.array_equal(hist2, hist_ref)
     assert np.array_equal(pr.interior(d[0]["p"].cpu().numpy()), pr.interior(ref[0]["p"]))
+
+
+@pytest.mark.parametrize("sweep", ["plain loads", "copies", "variable density", "FP32"])
+def test_every_sweep_takes_the_stall(lib, cuda, sweep, monkeypatch):
+    """The stall is taken by the half-sweep a solve runs anyway, whichever kernel
+    that is: arming it moves no solve to another kernel."""
+    if sweep == "copies":
+        monkeypatch.setenv("MF3D_SMALL_LEVEL_CELLS", "0")
+    pr = Problem(2, 1, 1, 16, 16, 16, ngrid=2, pl=1)
+    prm = pr.params(mg_itrsch=3, maxcy=3, eps=1e-12, lsm=int(sweep == "variable density"),
+                    precision=abi.MF3D_PREC_FP32 if sweep == "FP32" else abi.MF3D_PREC_FP64)
+    host = pr.block_fields(seed=9)
+    if prm.lsm:
+        for f, d in zip(host, pr.block_density(10)):
+            f["dens"] = d
+    proj = Projection(pr.descriptors(lib), prm, lib)
+    assert proj.tuning(1)["small_sweep"] == int(sweep != "copies")
+
+    def solve():
+        d = _dev(pr, host, cuda)
+        r = proj.newsolv_mg_device(d)
+        return r.history.tolist(), proj.launches, [f["p"].cpu() for f in d]
+
+    before = solve()
+    assert lib.mf3d_test_stall_copy(0, 16) == abi.MF3D_OK
+    with pytest.raises(RuntimeError, match="time limit"):
+        solve()
+    lib.mf3d_test_stall_copy(0, 0)
+    after = solve()
+    proj.close()
+    assert after[:2] == before[:2]
+    assert all(a.equal(b) for a, b in zip(after[2], before[2]))
