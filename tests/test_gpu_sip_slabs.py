@@ -6,9 +6,9 @@ that (a launch per hyperplane)."""
 import pytest
 
 from multiflow3d_b200 import abi
-from multiflow3d_b200.problems import Problem, WALL
+from multiflow3d_b200.problems import Problem, PERIODIC, WALL
 from multiflow3d_b200.solver import Projection
-from test_gpu_edges import run_both, assert_same
+from test_gpu_edges import run_both, assert_same, ragged_blocks
 from test_gpu_failures import _dev, _solve
 
 pytestmark = pytest.mark.gpu
@@ -148,3 +148,37 @@ def test_a_timeout_ends_the_call(lib, cuda):
     proj.close()
     assert st == abi.MF3D_E_TIMEOUT and "SIP" in abi.last_error(lib)
     assert stalled < whole / 100
+
+
+# lines past a CTA's shared memory with 12, 16 and more than 16 warps a CTA: the
+# rings are used again and again, across the slabs of a cluster
+RINGS = {
+    "12 warps": (48, 48, 48, 2),
+    "16 warps": (64, 64, 40, 2),
+    "16 warps, one segment": (20, 128, 60, 2),
+    "32 warps, many rounds": (200, 20, 60, 2),
+    "32 warps, short last slab": (32, 235, 40, 1),
+}
+
+
+@pytest.mark.parametrize("plane", sorted(RINGS))
+def test_rings_match_oracle(lib, oracle, cuda, plane):
+    nx, ny, nz, nswp = RINGS[plane]
+    pr = Problem(1, 1, 1, nx, ny, nz, bc=(WALL,) * 6, ngrid=1, pl=1, dx=0.013, dy=0.013, dz=0.013)
+    prm = pr.params(maxcy=3, eps=1e-9, solver=1, nswp=nswp)
+    o, g = run_both(lib, oracle, cuda, pr.descriptors(lib), pr.descriptors(oracle), pr.nblocks, prm,
+                    pr.block_fields(seed=50, fourier_modes=0))
+    assert_same(o, g, pr.pl)
+    rows = _launches(lib, cuda, (32, 32, 5), (1, 1, 1), 2) - _launches(lib, cuda, (32, 32, 5), (1, 1, 1), 1)
+    here = _launches(lib, cuda, (nx, ny, nz), (1, 1, 1), 2) - _launches(lib, cuda, (nx, ny, nz), (1, 1, 1), 1)
+    assert here == rows
+
+
+def test_rings_ragged_blocks(lib, oracle, cuda):
+    bc = (PERIODIC, PERIODIC, WALL, WALL, WALL, WALL)
+    args = ([40, 64, 21], 48, 70, 1 / 32, 1, bc, 51)
+    arr, blocks = ragged_blocks(lib, *args)
+    arr_o, _ = ragged_blocks(oracle, *args)
+    pr = Problem(1, 1, 1, 125, 48, 70, bc=bc, ngrid=1, pl=1)
+    o, g = run_both(lib, oracle, cuda, arr, arr_o, 3, pr.params(maxcy=3, eps=1e-9, solver=1, nswp=3), blocks)
+    assert_same(o, g, 1)
