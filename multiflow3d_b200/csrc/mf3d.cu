@@ -185,10 +185,13 @@ static inline int grid_of(long long n, int tpb) { return (int)((n + tpb - 1) / t
 
 // Every kernel of a solve is launched with programmatic stream
 // serialisation: its CTAs may be placed while the previous kernel on the
-// stream drains, and each kernel's first statement (pdl_wait) holds them
-// until that kernel has completed.  This removes the launch gap between the
-// dependent kernels of an iteration - most of the cost of the small coarse
-// levels.  The edges survive stream capture, so the solve graphs keep them.
+// stream drains or, where that one is a single wave, as soon as all its CTAs
+// run.  Each kernel's pdl_wait holds them until that kernel has completed;
+// ahead of it stand only reads of tables that the host uploaded (work lists,
+// descriptors, 1-D coefficients) and of the testing aid's flag.  This removes
+// the launch gap between the dependent kernels of an iteration - most of the
+// cost of the small coarse levels.  The edges survive stream capture, so the
+// solve graphs keep them.
 // MF3D_PDL=0 (read once) launches without the attribute, for comparison.
 static bool pdl_enabled() {
   static const bool on = [] {
@@ -235,8 +238,9 @@ static cudaError_t launch_cl(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 }
 
 // A cooperative launch (every CTA resident at once, for a kernel with grid
-// barriers), in plain stream order: no programmatic overlap with the kernels
-// around it, so no other grid holds the SMs its CTAs need.
+// barriers), in plain stream order: it starts after the kernel before it and
+// signals no dependents early (pdl_wait(0)), so no other grid holds the SMs its
+// CTAs need.
 template <typename... KArgs, typename... Args>
 static cudaError_t launch_coop(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                Args &&...args) {
@@ -2261,7 +2265,7 @@ static int autotune_level(mf3d_ctx *C, View &V, int g, bool time_new) {
       L.small = (v >> 3) & 1;
     } else if (time_new) {
       // candidates 0 .. kSweepSchedules-1: k_rbgs with that schedule;
-      // kSweepSchedules: k_rbgs_small (levels of 64 K to 4 M cells)
+      // kSweepSchedules: k_rbgs_small (levels of kTunedCells to 4 M cells)
       const long long cells = L.cells_sub[SUB_A];
       const bool small_ok = g > 1 && cells >= kTunedCells && cells <= (1LL << 22);
       const int n = kSweepSchedules + (small_ok ? 1 : 0);

@@ -94,7 +94,7 @@ template <typename T>
 __global__ void __launch_bounds__(MID_THREADS, MID_CTAS_PER_SM) k_mid_cycle(const MidPhase *__restrict__ phases,
                                                                              int nph, const int *__restrict__ act,
                                                                              MidBar *bar, int *__restrict__ err) {
-  pdl_wait();
+  pdl_wait(0);  // no early signal: no other grid's CTAs beside the grid barriers
   if (*(volatile const int *)err) return;  // an earlier wait gave up: the call is failing already
   // the phase's listed blocks: fine (and coarse) descriptors, item prefix,
   // the divisors that split a block's item index
