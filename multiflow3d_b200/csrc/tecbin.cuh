@@ -36,7 +36,10 @@ struct TbHead {  // the three framed header records
   int w[13];
 };
 
-__device__ int g_tecbin_err;  // first bad record + 1 (0: none)
+// first bad record + 1 (0: none): one for a device, so one decode at a time
+// holds it from its kernel to its answer (g_tecbin_lock)
+__device__ int g_tecbin_err;
+static std::mutex g_tecbin_lock[64];
 
 // Decode: cell record r -> out[f][r] for the 16 fields the reader keeps
 // (initial.for:718-733: p .. vwm, record fields 4..19); a null out[f] skips
@@ -155,6 +158,7 @@ int mf3d_tecbin_decode_device(const void *image, const mf3d_tecbin_info *info, d
   const long long nblk = (info->records + TB_CTA - 1) / TB_CTA;
   if (nblk > 0x7fffffffLL) { set_error("tecbin: too many records"); return MF3D_E_INVALID; }
   const unsigned *words = (const unsigned *)((const char *)image + info->data_offset);
+  std::lock_guard<std::mutex> hold(g_tecbin_lock[(unsigned)device % 64]);
   k_tecbin_decode<<<(unsigned)nblk, TB_CTA>>>(words, info->records, ptrs);
   // the blocking copy waits for the kernel; the flag is 0 between calls
   int bad = 0;

@@ -119,3 +119,34 @@ def test_device_decode_rejects_broken_framing(lib, cuda):
     st, _ = _decode(lib, cuda, bytes(data))
     assert st == abi.MF3D_E_INVALID
     assert b"record 77" in lib.mf3d_last_error()
+
+
+@pytest.mark.gpu
+def test_decodes_of_two_threads_do_not_mix(lib, cuda):
+    """One thread decodes a good image, another one with a broken record: each
+    call gets the answer of its own image."""
+    import threading
+    import torch
+    good = fixture_bytes()
+    bad = bytearray(good)
+    bad[52 + 160 * 9] ^= 1
+    info = abi.TecbinInfo()
+    assert lib.mf3d_tecbin_info_of(good, len(good), C.byref(info)) == 0
+    wrong = []
+
+    def decode(image, want):
+        dev = torch.from_numpy(np.frombuffer(bytes(image), dtype=np.uint8).copy()).to(cuda)
+        outs = [torch.empty(info.records, dtype=torch.float64, device=cuda) for _ in range(16)]
+        ptrs = (C.c_void_p * 16)(*[o.data_ptr() for o in outs])
+        torch.cuda.synchronize()
+        for _ in range(2000):
+            st = lib.mf3d_tecbin_decode_device(C.c_void_p(dev.data_ptr()), C.byref(info), ptrs, 0)
+            if st != want:
+                wrong.append((want, st))
+
+    threads = [threading.Thread(target=decode, args=a) for a in ((good, 0), (bad, abi.MF3D_E_INVALID))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, (len(wrong), wrong[:3])
