@@ -771,10 +771,12 @@ __global__ void __launch_bounds__(TD_THREADS) k_tdma_lines(const BlkLev *__restr
 // diagonal), 128^3: 4 V-cycles of the whole hierarchy 127 ms against 160.  With rhs'
 // formed by the recurrences' warp 1.56 ms; TW_CH = 4 1.48 ms.
 constexpr int TW_THREADS = 256, TW_CH = 8, TW_LINES = 32;
-// elements of shared memory (of T) for lmax lines of nmax cells
+// elements of shared memory (of T) for lmax lines of nmax cells.  The last
+// TW_CH are spare: the recurrences load ahead past a short line's coefficients
+// (not loading there, a test in front of the loop, costs 3 % of a solve).
 __host__ __device__ inline long long tw_elems(int lmax, int nmax, int coefs) {
   const long long ld = (nmax + 1) | 1;
-  return 11LL * lmax * ld + 4 * ld + 4 * lmax + coefs;
+  return 11LL * lmax * ld + 4 * ld + 4 * lmax + coefs + TW_CH;
 }
 template <typename T>
 __global__ void __launch_bounds__(TW_THREADS) k_tdma_wave(const BlkLev *__restrict__ bl, const int *__restrict__ blocks,
@@ -858,10 +860,10 @@ __global__ void __launch_bounds__(TW_THREADS) k_tdma_wave(const BlkLev *__restri
           const T *ar = rp + b * sl + lane * ld, *av = aa + b * sl + lane * ld;
           T *out = ph + b * sl + lane * ld;
           // batches of TW_CH cells, the next one's operands loaded beside the
-          // chain.  The last batch's load ahead reads past the line: with n >=
-          // TW_CH cells its at most n + TW_CH'th element of `lo` lies within
-          // the 2*(n+2) that begin with lo = ab, the array's last.  Shorter
-          // lines (a level of one or two planes) load nothing ahead.
+          // chain.  These loads reach past the line, to the (n + TW_CH)'th
+          // element of `lo` at most, and stay inside the allocation: lo = ab is
+          // followed by at and by the spare elements of tw_elems (a line of one
+          // or two cells needs three of them).
           T r[TW_CH], z[TW_CH], y[TW_CH];
           auto get = [&](int m0) {
 #pragma unroll
@@ -873,7 +875,7 @@ __global__ void __launch_bounds__(TW_THREADS) k_tdma_wave(const BlkLev *__restri
             }
           };
           const int nf = n / TW_CH * TW_CH;
-          if (nf > 0) get(0);
+          get(0);
           T c = g0[b * lmax + lane];
           for (int m0 = 0; m0 < nf; m0 += TW_CH) {
             T rr[TW_CH], zz[TW_CH], yy[TW_CH];

@@ -1231,7 +1231,7 @@ static int plane_tiles(const mf3d_ctx *C, const std::vector<PlaneExt> &ext, std:
 // slice of a diagonal is at most a warp's lanes and shared memory holds it
 // with the next one's staging (1-D coefficients only), else k_tdma_lines with
 // as many lines staged at a time as fit.
-constexpr size_t kTdSmem = 200 * 1024, kTwSmem = 220 * 1024;
+constexpr size_t kTdSmem = 200 * 1024, kTwSmem = 220 * 1024 + TW_CH * sizeof(double);
 static void td_shape(ViewLevel &L, int cl) {
   const size_t sz = L.td_fp64 ? 8 : 4;
   const int per = (L.td_numax + cl - 1) / cl;
