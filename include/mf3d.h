@@ -466,7 +466,8 @@ long long mf3d_field_exchange_map(const mf3d_block_desc *blocks, int nblocks, in
  * mf3d_test_stall_copy: on `device`, the next red-black half-sweep declares
  * `bytes` (1..65536) more on one CTA's first copy barrier than its copies
  * deliver; that CTA's bounded wait gives up after 2 s and the call returns
- * MF3D_E_TIMEOUT.  The copies themselves complete; 0 clears it.  With solver 1
+ * MF3D_E_TIMEOUT.  The copies themselves complete; 0 clears it.  A half-sweep
+ * with plain loads has no copies: it waits for the bytes alone.  With solver 1
  * the next launch of the substitutions takes it instead: one row segment
  * withholds its values, and the waits for them give up in the same way. */
 int mf3d_test_fail_alloc(long long after);

@@ -107,8 +107,10 @@ __device__ __forceinline__ void cell_coefs(const BlkLev &B, const Coef<T> &cf, i
 // slower there (11.0 against 11.4 solves/s at 256^3), the waiting CTAs
 // taking issue slots from the last wave.
 // 64x32x32 channel 1555 -> 1370 us a solve, 128^3 variable density 27.2 ->
-// 25.5 ms, 256^3 81.5 -> 80.1 ms.  One wave is taken as 4 CTAs an SM: with 6
-// 256^3 takes 80.9 ms, with 8 the 64-domain batch 311 against 298 ms.
+// 25.5 ms, 256^3 81.5 -> 80.7 ms.  One wave is taken as 4 CTAs on each of the
+// 148 SMs, whatever the kernel's occupancy (with fewer CTAs an SM the signal
+// comes when the last of them starts): with 6 256^3 takes 0.8 ms more, with 8
+// the 64-domain batch 311 against 298 ms.
 constexpr unsigned kPdlCtas = 592;
 __device__ __forceinline__ bool pdl_one_wave() { return gridDim.x * gridDim.y <= kPdlCtas; }
 // ctas: what one wave holds of the kernel (2*kPdlCtas: 8 light CTAs an SM)

@@ -1261,10 +1261,10 @@ static void tdma_relax(mf3d_ctx *C, View &V, ViewLevel &L, int q) {
 
 // Line relaxation (mg_itrsch 2) on level g: room for every listed block's
 // TDMA factors (six arrays of its cells, k_tdma_factor), pointed to from its
-// table entry, and the shape of k_tdma_lines.  A block whose diagonals hold
-// fewer than 32 lines is one CTA; larger ones take a cluster of 4 CTAs or
-// more (below), each CTA owning a slice of at least 8 line positions of
-// every diagonal.
+// table entry, and the kernel and its shape (td_shape: k_tdma_wave where a
+// slice fits, else k_tdma_lines).  A block whose diagonals hold fewer than 32
+// lines is one CTA; larger ones take a cluster of 4 CTAs or more (below), each
+// CTA owning a slice of at least 8 line positions of every diagonal.
 static int tdma_layout(mf3d_ctx *C, View &V, int g, std::vector<BlkLev> &tab) {
   ViewLevel &L = V.lv[g];
   const int nb = (int)V.blk.size();

@@ -1293,7 +1293,9 @@ __global__ void __launch_bounds__(RW_TX *RW_RJ) k_calmas4(const BlkFld *__restri
 // 256^3 in 8 blocks: 267 us a component with six IEEE divisions a cell, every
 // operand loaded anew and none ahead; 193 us as it stands for 3 CTAs an SM,
 // 168 for 4 (4.8 TB/s; a stage 690 and 635 us; 5: 874, the loads ahead spill; 4
-// without them: 751).
+// without them: 751).  Those are spacings of powers of two (MODE 2); others
+// (MODE 1) hold six reciprocals more and take 3 CTAs: at a spacing of 0.0113 a
+// stage takes 894 us with 3, 932 with 2, 1287 with 4.
 template <int COMP>
 struct Rk2Plane {  // what a plane adds to the march at (i, j): C at the plane above, this plane's neighbours
   double ct, cw, ce, cs, cn;  // C(k+1), C(i-1), C(i+1), C(j-1), C(j+1)
@@ -1537,7 +1539,9 @@ __device__ __forceinline__ double weno5(double v1, double v2, double v3, double 
 // evaluation on selected differences (a warp holds both signs), and the
 // quotients by h, h*h and the weights' sum need no division each (quo).
 // 128^3 in 8 blocks: 268 us a component before, 137 for 2 CTAs an SM; a stage
-// 531 us, 447 for 4 (3: 494, 5: 456, 6: 501).
+// 531 us, 447 for 4 (3: 494, 5: 456, 6: 501), spacings of powers of two.  Other
+// spacings (MODE 1) have 3: at 0.0113 a stage takes 550 us, 577 with 2, 506
+// with 4, which is slower on one block of 40^3 (230 against 224).
 template <int COMP, int MODE>
 __device__ __forceinline__ double rkw_cell(const double *U, const double *V, const double *W, const double *OO,
                                            const double *VIS, const long long *st3, const int *fx, const int *lim,

@@ -188,8 +188,8 @@ __global__ void k_sip_sum(const double *__restrict__ part, int n, SipCtl *__rest
 
 // Forward substitution on hyperplane h (sipsol.for:149-157).  `run` is loaded
 // beside the operands and looked at before the store: a launch is a chain of
-// loads, and one more ahead of them cost 0.6 us of 2.3 (96x96x64: 27.8 ms for
-// 6 calls of 4 sweeps, 35.1 with it).
+// loads, and one more ahead of them cost 0.6 us of 2.9 (96x96x64, 3 calls of 4
+// sweeps: 17.9 ms with it, 13.9 without).
 __global__ void k_sip_forward(const SipBlk *__restrict__ sb, const Tile *__restrict__ tiles, int h,
                               const SipCtl *__restrict__ ctl) {
   pdl_wait();
@@ -259,7 +259,7 @@ __global__ void k_sip_backward(const SipBlk *__restrict__ sb, const BlkLev *__re
 // each four steps of a shuffle and four dependent FP64 operations; DRAM and
 // issue slots are nearly idle.  Eight blocks of 32^3: 70 us a sweep (cold),
 // against 312 us for one CTA per block with two barriers per hyperplane and
-// the operands one step ahead; the solve of 50 calls of 4 sweeps 65.3 -> 18.6
+// the operands one step ahead; the solve of 50 calls of 4 sweeps 65.2 -> 17.2
 // ms.  A barrier per hyperplane over a cluster with operands by cp.async four
 // steps ahead took 180 us; the rings' fences (RING) cost 8 % of the solve.
 constexpr long long kSipEmpty = 0x7ff45a5a5a5a5a5aLL;
@@ -659,7 +659,6 @@ constexpr int kSipSlabs = 8;  // CTAs per block of k_sip_subst at most (portable
 // hold a block's warps.  warps: per CTA.
 static int sip_slabs(const std::vector<SipBlk> &hb, int nsm, int W, int &warps) {
   long long need = 1, want = 1;
-
   for (const auto &b : hb) {
     const long long nseg = (b.nx + 31) / 32, fit = W / nseg;
     if (!fit) return 0;
