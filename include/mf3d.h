@@ -468,8 +468,8 @@ long long mf3d_field_exchange_map(const mf3d_block_desc *blocks, int nblocks, in
  * deliver; that CTA's bounded wait gives up after 2 s and the call returns
  * MF3D_E_TIMEOUT.  The copies themselves complete; 0 clears it.  A half-sweep
  * with plain loads has no copies: it waits for the bytes alone.  With solver 1
- * the next launch of the substitutions takes it instead: one row segment
- * withholds its values, and the waits for them give up in the same way. */
+ * the next launch in which row segments wait for one another takes it instead:
+ * one withholds its values, and the waits for them give up in the same way. */
 int mf3d_test_fail_alloc(long long after);
 int mf3d_test_stall_copy(int device, int bytes);
 

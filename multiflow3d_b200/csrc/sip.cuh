@@ -156,11 +156,10 @@ __global__ void __launch_bounds__(RW_TX *RW_RJ) k_sip_residual(const SipBlk *__r
 // The per-CTA sums added in index order by one CTA (a fixed tree), then
 // the stopping test of sipsol.for on the sum.  After a wait of the
 // substitutions gave up nothing runs any more: the call has failed.
-__global__ void k_sip_sum(const double *__restrict__ part, int n, SipCtl *__restrict__ ctl,
-                          const int *__restrict__ err) {
+__global__ void k_sip_sum(const double *__restrict__ part, int n, SipCtl *__restrict__ ctl, const int *err) {
   pdl_wait();
   __shared__ double s[1024];
-  const int go = *err == ERR_SIP_WAIT ? 0 : ctl->next;
+  const int go = *(volatile const int *)err == ERR_SIP_WAIT ? 0 : ctl->next;
   double v = 0.0;
   if (go)
     for (int q = threadIdx.x; q < n; q += blockDim.x) v = v + part[q];
